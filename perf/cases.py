@@ -17,13 +17,15 @@ the simulation its state (device arrays in original order; the drop-in's
 caller restores its own buffers), advances it by ``steps`` timesteps and
 takes it back whole, in original particle order, as a program does that
 couples the simulation to another one or branches trajectories from a state.
-Twelve steps or more take in the neighbour-list rebuilds of a running
-simulation, about one per eight steps.  Positions come back unwrapped
-(position + crossings times box length), as a program that tracks particles
-or membranes uses them.  The Morse force ends at its cut-off with a jump, so
-a pair there counts or not by the last bit of a position; the scene with tens
-of thousands of aggregating vertices returns deformation and aggregation
-force as one sum, in which that is lost.
+Two states are handed over in turn, so that every pass of the library-owned
+simulations re-sorts and rebuilds the neighbour lists once, in its first
+step: one rebuild per 12 to 16 steps (a running suspension needs one per 8
+to 10).  Positions come back unwrapped (position + crossings times box
+length), as a program that tracks particles or membranes uses them.  The
+Morse force ends at its cut-off with a jump, so a pair there counts or not by
+the last bit of a position; the scene with tens of thousands of aggregating
+vertices returns deformation and aggregation force as one sum, in which that
+is lost.
 
 ``exact`` is the method in 64 bits, in plain torch: integration, densities,
 SDPD pair forces with their Philox pair noise, wall repulsion and no-slip
@@ -189,12 +191,13 @@ def _configs(case):
     return _scene(tuple(sorted((k, v) for k, v in case.items() if k not in ("name", "api", "noise", "steps"))))
 
 
-def _inputs(case, seed):
+def _inputs(case, seed, which=0):
     """Per system of the case: its configuration with the fluid displaced
-    from the lattice, and the thermal velocities of its moving particles."""
+    from the lattice, and the thermal velocities of its moving particles
+    (`which`: the first or the second of the states handed over in turn)."""
     out = []
     for k, cfg in enumerate(_configs(case)):
-        rng = np.random.default_rng([seed, k])
+        rng = np.random.default_rng([seed, k, which])
         fl, me = cfg.n_b1 + cfg.n_b2, cfg.n_cell_start
         coor = cfg.coor.copy()
         coor[fl:me] += (rng.random((cfg.n_fluid, 3), np.float32) - np.float32(0.5)) * np.float32(0.2 * DX)
@@ -217,37 +220,41 @@ def _inputs(case, seed):
 _CELLS = ("area", "vol", "defforce", "aggforce", "trinordir", "tricenter", "pararea")
 
 
+def _lengths(cfg):
+    """Box lengths on the periodic axes (0 elsewhere)."""
+    return torch.as_tensor((cfg.bbox[1::2] - cfg.bbox[0::2]) * np.float32([cfg.pmask >> a & 1 for a in range(3)]))[None]
+
+
 def _ptr(t):
     return C.c_void_p(t.data_ptr() if t is not None else 0)
 
 
 def prepare(case, seed):
-    inputs = _inputs(case, seed)
-    cfgs = [c for c, _ in inputs]
-    lengths = torch.cat([torch.tensor((c.bbox[1::2] - c.bbox[0::2]) * [c.pmask >> a & 1 for a in range(3)],
-                                      dtype=torch.float32).expand(c.n if case["api"] == "ensemble" else 1, 3)
-                         for c in cfgs]).to(DEVICE)
-    state = dict(case=case, lengths=lengths)
+    cfgs = _configs(case)
+    z = lambda *shape, dt=torch.float32: torch.zeros(shape, dtype=dt, device=DEVICE)
     if case["api"] == "dropin":
-        cfg, vel = inputs[0]
-        state["system"] = ps = ParticleSystem(cfg, device=DEVICE, noise=case["noise"])
+        (cfg, vel), = _inputs(case, seed)
+        ps = ParticleSystem(cfg, device=DEVICE, noise=case["noise"])
         ps.set_state(vel=vel)
-        state["start"] = {k: ps.d[k].clone() for k in ("TotalCoor", "Velrhop", "VelHalf", "TotalForce", "SortPart", "nThroBound")}
-        return state
-    if case["api"] == "ensemble":
-        fs = Ensemble(cfgs, noise=case["noise"])
-    else:
-        fs = FusedSystem(cfgs[0], noise=case["noise"], graph=case["api"] == "captured")
+        keep = ("TotalCoor", "Velrhop", "VelHalf", "TotalForce", "SortPart", "nThroBound")
+        return dict(case=case, system=ps, lengths=_lengths(cfgs[0]).to(DEVICE), start={k: ps.d[k].clone() for k in keep})
     n, ncell = sum(c.n for c in cfgs), sum(c.ncell for c in cfgs)
     ntri, ncp = sum(c.ntri for c in cfgs), sum(c.ncp for c in cfgs)
-    z = lambda *shape, dt=torch.float32: torch.zeros(shape, dtype=dt, device=DEVICE)
+    if case["api"] == "ensemble":
+        fs = Ensemble(cfgs, noise=case["noise"])
+        lengths = torch.cat([_lengths(c).expand(c.n, 3) for c in cfgs]).to(DEVICE)
+    else:
+        fs = FusedSystem(cfgs[0], noise=case["noise"], graph=case["api"] == "captured")
+        lengths = _lengths(cfgs[0]).to(DEVICE)
     up = lambda arrays: torch.as_tensor(np.concatenate(arrays), device=DEVICE)
-    state["start"] = [up([c.coor for c in cfgs]), up([v for _, v in inputs]), up([c.velhalf for c in cfgs]), z(n, 3),
-                      z(n, 3, dt=torch.int32)]
-    state.update(system=fs, pos=z(n, 3), vel=z(n, 3), rho=z(n), press=z(n), force=z(n, 3),
-                 nthro=z(n, 3, dt=torch.int32),
-                 cells=dict(zip(_CELLS, (z(ncell), z(ncell), z(ncp, 3), z(ncp, 3), z(ntri, 3), z(ntri, 3), z(ncp)))) if ncell else {})
-    return state
+    start = []
+    for which in (0, 1):
+        inputs = _inputs(case, seed, which)
+        start.append([up([c.coor for c, _ in inputs]), up([v for _, v in inputs]), up([c.velhalf for c in cfgs]), z(n, 3),
+                      z(n, 3, dt=torch.int32)])
+    cells = dict(zip(_CELLS, (z(ncell), z(ncell), z(ncp, 3), z(ncp, 3), z(ntri, 3), z(ntri, 3), z(ncp)))) if ncell else {}
+    return dict(case=case, system=fs, lengths=lengths, start=start, passes=0, pos=z(n, 3), vel=z(n, 3), rho=z(n), press=z(n),
+                force=z(n, 3), nthro=z(n, 3, dt=torch.int32), cells=cells)
 
 
 def _membrane(case, cells):
@@ -280,7 +287,8 @@ def run(state):
                 area=d["Area"], vol=d["Vol"], defforce=d["DefForce"], aggforce=d["AggForce"], trinordir=d["TriNorDir"],
                 tricenter=d["TriCenter"], pararea=d["ParArea"])))
         return out
-    _lib.call("gc_fused_load", s.h, *[_ptr(t) for t in state["start"]], 1)
+    _lib.call("gc_fused_load", s.h, *[_ptr(t) for t in state["start"][state["passes"] % 2]], 1)
+    state["passes"] += 1
     s.step(case["steps"], 1)
     _lib.call("gc_fused_store", s.h, _ptr(state["pos"]), _ptr(state["vel"]), _ptr(state["rho"]), _ptr(state["press"]),
               _ptr(state["force"]), _ptr(None), _ptr(state["nthro"]), 1)

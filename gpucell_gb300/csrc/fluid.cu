@@ -2,11 +2,12 @@
 // integrator stages, periodic wrap, density, equation of state, the SDPD
 // pair force, wall repulsion, body force and the no-slip wall velocity.
 //
-// These are the reference-structured FP32 kernels behind the drop-in
-// boundary: one kernel per entry point, one thread per slot, a 27-cube sweep
-// over the caller's begin/end table for every neighbour pass, float3/float4
-// arrays in the caller's layout.  Particle type is decided from the original
-// id in d_sortpart (src/Particle.cu:432-435).
+// These are the FP32 kernels behind the drop-in boundary: one kernel per
+// entry point on the caller's arrays (float3/float4, slot order), no state
+// kept from one call to the next.  The neighbour passes sweep the 27 cubes of
+// the caller's begin/end table, one block per cube (sweep.cuh); the others run
+// one thread per slot.  Particle type is decided from the original id in
+// d_sortpart (src/Particle.cu:432-435).
 //
 // The formulas (pinned because GPUCell's kernel bodies are absent):
 //   density   rho_i = m (W(0) + sum_j W_ij), j over Bound2, fluid, membrane;
@@ -25,29 +26,13 @@
 //             v_presc = the wall's VelHalf (zero unless the caller sets it)
 //   integrator Groot & Warren (1997) modified velocity-Verlet with lambda = VVsigma
 #include "gc_internal.cuh"
+#include "sweep.cuh"
 
 namespace {
 
-// Visits every slot j in the 27 cubes around cube c (periodic axes wrap,
-// wall axes stop at the edge).  Cube counts per periodic axis are >= 3, so
-// no cube is visited twice.
-template <class Fn>
-__device__ __forceinline__ void sweep27(const GcParams& p, int3 c, const int2* __restrict__ bec, Fn&& fn) {
-    for (int dz = -1; dz <= 1; ++dz) {
-        int z = cube_step(c.z, dz, 2, p.g);
-        if (z < 0) continue;
-        for (int dy = -1; dy <= 1; ++dy) {
-            int y = cube_step(c.y, dy, 1, p.g);
-            if (y < 0) continue;
-            for (int dx = -1; dx <= 1; ++dx) {
-                int x = cube_step(c.x, dx, 0, p.g);
-                if (x < 0) continue;
-                int2 be = bec[cube_key(x, y, z, p.g)];
-                for (int j = be.x; j < be.y; ++j) fn(j);
-            }
-        }
-    }
-}
+// Smallest normal number: squared distances below it (particles within 1e-19
+// of each other) count as zero, and rsqrt_ftz takes normal arguments only.
+constexpr float kTiny = 1.17549435e-38f;
 
 // K2 -- r += dt v + dt^2/2 F/m for fluid and membrane particles.
 __global__ void k_update_coor(int n, GcParams p, const int* __restrict__ sortpart, const float3* __restrict__ force,
@@ -91,24 +76,27 @@ __global__ void k_periodic(int n, GcParams p, const int* __restrict__ sortpart, 
     nthro[i] = t;
 }
 
-// K8 -- kernel-sum density of fluid and membrane particles.
-__global__ void k_density(int n, GcParams p, const float3* __restrict__ coor, float4* __restrict__ velrhop,
-                          const int3* __restrict__ cc, const int* __restrict__ sortpart, const int2* __restrict__ bec) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (!is_mobile((unsigned)sortpart[i], p)) return;
-    float3 xi = coor[i];
-    float sum = p.w0;
-    sweep27(p, cc[i], bec, [&](int j) {
-        if (j == i) return;
-        float3 d = min_image(xi, coor[j], p.g);
-        float r2 = norm2_rn(d);
-        if (r2 >= p.rc2) return;
-        if (!is_sdpd((unsigned)sortpart[j], p)) return;
-        sum += wendland_w(sqrtf(r2), p);
-    });
-    velrhop[i].w = p.mass * sum;
-}
+// K8 -- kernel-sum density of fluid and membrane particles (the particle's
+// own share W(0) comes with its own entry among the candidates).
+struct DensityOp {
+    float4* velrhop;
+    static constexpr int kBlocks = 8;   // resident blocks the registers are cut to
+    static constexpr bool kExact = false;
+    struct Extra {};
+    struct Self {};
+    struct Acc { float sum; };
+    __device__ float cut2(const GcParams& p) const { return p.rc2; }
+    __device__ bool active(unsigned id, const GcParams& p) const { return is_mobile(id, p); }
+    __device__ bool keep(unsigned id, const GcParams& p) const { return is_sdpd(id, p); }
+    __device__ void idle(int) const {}
+    __device__ void begin(Acc& a, Self&, int, unsigned, bool, const GcParams&) const { a.sum = 0.f; }
+    __device__ void stage(Extra&, int, int, const GcParams&) const {}
+    __device__ void pair(Acc& a, const Self&, const Extra&, int, unsigned, float3, float r2, const GcParams& p) const {
+        a.sum += wendland_w(r2 < kTiny ? 0.f : r2 * rsqrt_ftz(r2), p);
+    }
+    __device__ void reduce(Acc& a) const { a.sum = gcsweep::lane_sum(a.sum); }
+    __device__ void finish(const Acc& a, const Self&, int i, const GcParams& p) const { velrhop[i].w = p.mass * a.sum; }
+};
 
 // K9 -- predictor: VelHalf = v + dt/2 F/m, v <- v + lambda dt F/m.
 __global__ void k_predict(int n, GcParams p, const int* __restrict__ sortpart, float4* __restrict__ velrhop,
@@ -127,37 +115,49 @@ __global__ void k_predict(int n, GcParams p, const int* __restrict__ sortpart, f
 }
 
 // K10 -- no-slip velocity of Bound2 wall particles.
-__global__ void k_bound2vel(int n, GcParams p, const float3* __restrict__ coor, float4* __restrict__ velrhop,
-                            const float3* __restrict__ velhalf, const int3* __restrict__ cc,
-                            const int* __restrict__ sortpart, const int2* __restrict__ bec) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (ptype((unsigned)sortpart[i], p) != PT_B2) return;
-    float3 xi = coor[i];
-    float3 num = f3(0.f, 0.f, 0.f);
-    float den = 0.f;
-    sweep27(p, cc[i], bec, [&](int j) {
-        float3 d = min_image(xi, coor[j], p.g);
-        float r2 = norm2_rn(d);
-        if (r2 >= p.rc2) return;
-        if (!is_mobile((unsigned)sortpart[j], p)) return;
-        float w = wendland_w(sqrtf(r2), p);
-        float4 vj = velrhop[j];
-        num += w * f3(vj.x, vj.y, vj.z);
-        den += w;
-    });
-    float3 vw = velhalf ? velhalf[i] : f3(0.f, 0.f, 0.f);
-    float4 v = velrhop[i];
-    if (den > 0.f) {
-        float inv = 1.f / den;
-        v.x = 2.f * vw.x - num.x * inv;
-        v.y = 2.f * vw.y - num.y * inv;
-        v.z = 2.f * vw.z - num.z * inv;
-    } else {
-        v.x = vw.x; v.y = vw.y; v.z = vw.z;
+struct Bound2VelOp {
+    float4* velrhop;
+    const float3* velhalf;
+    static constexpr int kBlocks = 6;   // resident blocks the registers are cut to
+    static constexpr bool kExact = false;
+    struct Extra { float3 v[gcsweep::kCap]; };
+    struct Self {};
+    struct Acc { float3 num; float den; };
+    __device__ float cut2(const GcParams& p) const { return p.rc2; }
+    __device__ bool active(unsigned id, const GcParams& p) const { return ptype(id, p) == PT_B2; }
+    __device__ bool keep(unsigned id, const GcParams& p) const { return is_mobile(id, p); }
+    __device__ void idle(int) const {}
+    __device__ void begin(Acc& a, Self&, int, unsigned, bool, const GcParams&) const {
+        a.num = f3(0.f, 0.f, 0.f);
+        a.den = 0.f;
     }
-    velrhop[i] = v;
-}
+    __device__ void stage(Extra& e, int q, int j, const GcParams&) const {
+        const float4 v = velrhop[j];
+        e.v[q] = f3(v.x, v.y, v.z);
+    }
+    __device__ void pair(Acc& a, const Self&, const Extra& e, int q, unsigned, float3, float r2, const GcParams& p) const {
+        const float w = wendland_w(r2 < kTiny ? 0.f : r2 * rsqrt_ftz(r2), p);
+        a.num += w * e.v[q];
+        a.den += w;
+    }
+    __device__ void reduce(Acc& a) const {
+        a.num = f3(gcsweep::lane_sum(a.num.x), gcsweep::lane_sum(a.num.y), gcsweep::lane_sum(a.num.z));
+        a.den = gcsweep::lane_sum(a.den);
+    }
+    __device__ void finish(const Acc& a, const Self&, int i, const GcParams&) const {
+        const float3 vw = velhalf ? velhalf[i] : f3(0.f, 0.f, 0.f);
+        float4 v = velrhop[i];
+        if (a.den > 0.f) {
+            const float inv = 1.f / a.den;
+            v.x = 2.f * vw.x - a.num.x * inv;
+            v.y = 2.f * vw.y - a.num.y * inv;
+            v.z = 2.f * vw.z - a.num.z * inv;
+        } else {
+            v.x = vw.x; v.y = vw.y; v.z = vw.z;
+        }
+        velrhop[i] = v;   // walls only: no other block stages this slot's velocity
+    }
+};
 
 // K11 -- equation of state.
 __global__ void k_eos(int n, GcParams p, const int* __restrict__ sortpart, const float4* __restrict__ velrhop,
@@ -173,78 +173,102 @@ __global__ void k_eos(int n, GcParams p, const int* __restrict__ sortpart, const
 }
 
 // K12 -- SDPD pair force; writes the force of every slot (zero for walls).
-__global__ void k_sdpd(int n, GcParams p, const float3* __restrict__ coor, const float4* __restrict__ velrhop,
-                       const int3* __restrict__ cc, const int* __restrict__ sortpart, const int2* __restrict__ bec,
-                       float3* __restrict__ force, const float* __restrict__ press) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    unsigned id = (unsigned)sortpart[i];
-    if (!is_mobile(id, p)) {
-        force[i] = f3(0.f, 0.f, 0.f);
-        return;
+// A candidate's velocity, 1/d and P/d^2 are staged with its position.  The
+// pair terms are gathered into one coefficient along d = x_i - x_j (pressure
+// and the e e^T parts of the viscous and random forces, e = d/r folded in as
+// 1/r^2), one along v_ij and one along xi_ij, as in the fused step.
+template <bool NOISE>
+struct SdpdOp {
+    const float4* velrhop;
+    const float* press;
+    float3* force;
+    static constexpr int kBlocks = 6;   // resident blocks the registers are cut to
+    static constexpr bool kExact = false;
+    struct Extra { float4 v[gcsweep::kCap]; float pt[gcsweep::kCap]; };
+    struct Self { float3 v; float inv_d, pt; unsigned id; };
+    struct Acc { float3 f; };
+    __device__ float cut2(const GcParams& p) const { return p.rc2; }
+    __device__ bool active(unsigned id, const GcParams& p) const { return is_mobile(id, p); }
+    __device__ bool keep(unsigned id, const GcParams& p) const { return is_sdpd(id, p); }
+    __device__ void idle(int i) const { force[i] = f3(0.f, 0.f, 0.f); }
+    __device__ void begin(Acc& a, Self& s, int i, unsigned id, bool act, const GcParams& p) const {
+        a.f = f3(0.f, 0.f, 0.f);
+        if (!act) return;
+        const float4 v = velrhop[i];
+        const float d = v.w * p.inv_mass;
+        s.v = f3(v.x, v.y, v.z);
+        s.inv_d = 1.f / d;
+        s.pt = press[i] / (d * d);
+        s.id = id;
     }
-    float3 xi = coor[i];
-    float4 vi = velrhop[i];
-    float di = vi.w * p.inv_mass;
-    float pi_term = press[i] / (di * di);
-    bool noise = p.noise_pref > 0.f;
-    float3 f = f3(0.f, 0.f, 0.f);
-    sweep27(p, cc[i], bec, [&](int j) {
-        if (j == i) return;
-        float3 d = min_image(xi, coor[j], p.g);
-        float r2 = norm2_rn(d);
-        if (r2 >= p.rc2) return;
-        unsigned idj = (unsigned)sortpart[j];
-        if (!is_sdpd(idj, p)) return;
-        float r = sqrtf(r2);
-        float F = wendland_f(r, p);
-        float4 vj = velrhop[j];
-        float dj = vj.w * p.inv_mass;
-        float cons = (pi_term + press[j] / (dj * dj)) * F;
-        f += cons * d;
-        if (r2 <= 0.f) return;
-        float inv_r = 1.f / r;
-        float3 e = inv_r * d;
-        float3 vij = f3(vi.x - vj.x, vi.y - vj.y, vi.z - vj.z);
-        float ev = dot3(e, vij);
-        float fdd = F / (di * dj);
-        f -= fdd * (p.visA * vij + (p.visB * ev) * e);
-        if (noise) {
+    __device__ void stage(Extra& e, int q, int j, const GcParams& p) const {
+        const float4 v = velrhop[j];
+        const float d = v.w * p.inv_mass;
+        e.v[q] = make_float4(v.x, v.y, v.z, 1.f / d);
+        e.pt[q] = press[j] / (d * d);
+    }
+    __device__ void pair(Acc& a, const Self& s, const Extra& e, int q, unsigned idj, float3 d, float r2,
+                         const GcParams& p) const {
+        if (r2 < kTiny) return;   // the particle itself; coincident particles exert no force
+        const float4 vj = e.v[q];
+        const float inv_r = rsqrt_ftz(r2), ir2 = inv_r * inv_r;
+        const float F = wendland_f(r2 * inv_r, p);
+        const float3 vij = f3(s.v.x - vj.x, s.v.y - vj.y, s.v.z - vj.z);
+        const float fdd = F * (s.inv_d * vj.w);
+        float cd = (s.pt + e.pt[q]) * F - (fdd * p.visB) * dot3(d, vij) * ir2;
+        a.f += (-fdd * p.visA) * vij;
+        if constexpr (NOISE) {
             // a pair at the cut-off can give F a rounding-sized negative value: no noise then
-            float q = fdd > 0.f ? sqrtf(p.noise_pref * fdd) : 0.f;
-            float3 xi_ = pair_noise(id, idj, p);
-            float exi = dot3(e, xi_);
-            f += q * (p.sqrtA * xi_ + ((p.sqrtAB - p.sqrtA) * exi) * e);
+            const float qq = p.noise_pref * fdd;
+            float n = qq >= kTiny ? qq * rsqrt_ftz(qq) : 0.f;
+            n = s.id < idj ? n : -n;   // the pair sign of xi_ij
+            const float3 xi = pair_noise_unsigned(s.id, idj, p);
+            cd += (n * (p.sqrtAB - p.sqrtA)) * dot3(d, xi) * ir2;
+            a.f += (n * p.sqrtA) * xi;
         }
-    });
-    force[i] = f;
-}
+        a.f += cd * d;
+    }
+    __device__ void reduce(Acc& a) const {
+        a.f = f3(gcsweep::lane_sum(a.f.x), gcsweep::lane_sum(a.f.y), gcsweep::lane_sum(a.f.z));
+    }
+    __device__ void finish(const Acc& a, const Self&, int i, const GcParams&) const { force[i] = a.f; }
+};
 
 // K13 -- repulsion of fluid and membrane particles by Bound1 walls.
-__global__ void k_repulsion(int n, GcParams p, const float3* __restrict__ coor, const int3* __restrict__ cc,
-                            const int* __restrict__ sortpart, const int2* __restrict__ bec,
-                            float3* __restrict__ force) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (!is_mobile((unsigned)sortpart[i], p)) return;
-    float3 xi = coor[i];
-    float3 f = f3(0.f, 0.f, 0.f);
-    bool any = false;
-    sweep27(p, cc[i], bec, [&](int j) {
-        float3 d = min_image(xi, coor[j], p.g);
-        float r2 = norm2_rn(d);
-        if (r2 >= p.rep_r0sq || r2 <= 0.f) return;
-        if (ptype((unsigned)sortpart[j], p) != PT_B1) return;
-        float q2 = p.rep_r0sq / r2;
-        float q4 = q2 * q2;
-        float q12 = q4 * q4 * q4;
-        f += (p.rep_D * (q12 - q4) / r2) * d;
-        any = true;
-    });
-    if (any) {
-        float3 t = force[i];
-        force[i] = t + f;
+struct RepulsionOp {
+    float3* force;
+    static constexpr int kBlocks = 8;   // resident blocks the registers are cut to
+    static constexpr bool kExact = false;
+    struct Extra {};
+    struct Self {};
+    struct Acc { float3 f; };
+    __device__ float cut2(const GcParams& p) const { return p.rep_r0sq; }
+    __device__ bool active(unsigned id, const GcParams& p) const { return is_mobile(id, p); }
+    __device__ bool keep(unsigned id, const GcParams& p) const { return ptype(id, p) == PT_B1; }
+    __device__ void idle(int) const {}
+    __device__ void begin(Acc& a, Self&, int, unsigned, bool, const GcParams&) const { a.f = f3(0.f, 0.f, 0.f); }
+    __device__ void stage(Extra&, int, int, const GcParams&) const {}
+    __device__ void pair(Acc& a, const Self&, const Extra&, int, unsigned, float3 d, float r2, const GcParams& p) const {
+        if (r2 <= 0.f) return;
+        const float q2 = p.rep_r0sq / r2, q4 = q2 * q2, q12 = q4 * q4 * q4;
+        a.f += (p.rep_D * (q12 - q4) / r2) * d;
     }
+    __device__ void reduce(Acc& a) const {
+        a.f = f3(gcsweep::lane_sum(a.f.x), gcsweep::lane_sum(a.f.y), gcsweep::lane_sum(a.f.z));
+    }
+    __device__ void finish(const Acc& a, const Self&, int i, const GcParams&) const {
+        if (a.f.x != 0.f || a.f.y != 0.f || a.f.z != 0.f) force[i] += a.f;
+    }
+};
+
+template <class Op>
+int launch_sweep(const Op& op, int n, const GcParams& p, const float* coor, const int* sortpart, const int* bec,
+                 cudaStream_t st, const char* what) {
+    const int K = p.g.ncells, per = gcsweep::cubes_per_block(n, K);
+    gcsweep::k_sweep<<<gc_blocks(K, per), gcsweep::kBlock, 0, st>>>(K, per, p, op, (const float3*)coor, sortpart,
+                                                                    (const int2*)bec);
+    GC_CHECK_LAUNCH(what);
+    return GC_OK;
 }
 
 // K14 -- body force in x on fluid and membrane particles.
@@ -278,24 +302,44 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
     return z ^ (z >> 31);
 }
 
-__global__ void k_nbstats(int n, GcParams p, const float3* __restrict__ coor, const int* __restrict__ sortpart,
-                          const int2* __restrict__ bec, int* __restrict__ count, unsigned long long* __restrict__ hash) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float3 xi = coor[i];
-    int3 c = make_int3(cube_coord(xi.x, 0, p.g), cube_coord(xi.y, 1, p.g), cube_coord(xi.z, 2, p.g));
-    int cnt = 0;
-    unsigned long long h = 0;
-    sweep27(p, c, bec, [&](int j) {
-        if (j == i) return;
-        float3 d = min_image(xi, coor[j], p.g);
-        if (norm2_rn(d) >= p.rc2) return;
-        ++cnt;
-        h += mix64((unsigned long long)(unsigned)sortpart[j]);
-    });
-    count[i] = cnt;
-    hash[i] = h;
-}
+// Number and id checksum of every slot's neighbours.  The sweep marks with a
+// slightly larger cut-off and the pair function applies the predicate of the
+// oracle, bit for bit.
+struct NeighborOp {
+    int* count;
+    unsigned long long* hash;
+    static constexpr int kBlocks = 8;   // resident blocks the registers are cut to
+    static constexpr bool kExact = true;
+    struct Extra {};
+    struct Self { unsigned id; };
+    struct Acc { int cnt; unsigned long long h; };
+    __device__ float cut2(const GcParams& p) const { return p.rc2 * 1.00001f; }
+    __device__ bool active(unsigned, const GcParams&) const { return true; }
+    __device__ bool keep(unsigned, const GcParams&) const { return true; }
+    __device__ void idle(int) const {}
+    __device__ void begin(Acc& a, Self& s, int, unsigned id, bool, const GcParams&) const {
+        a.cnt = 0;
+        a.h = 0;
+        s.id = id;
+    }
+    __device__ void stage(Extra&, int, int, const GcParams&) const {}
+    __device__ void pair(Acc& a, const Self& s, const Extra&, int, unsigned idj, float3, float r2, const GcParams& p) const {
+        if (r2 >= p.rc2 || idj == s.id) return;
+        ++a.cnt;
+        a.h += mix64((unsigned long long)idj);
+    }
+    __device__ void reduce(Acc& a) const {
+#pragma unroll
+        for (int o = gcsweep::kLanes / 2; o; o >>= 1) {
+            a.cnt += __shfl_xor_sync(0xffffffffu, a.cnt, o, gcsweep::kLanes);
+            a.h += __shfl_xor_sync(0xffffffffu, a.h, o, gcsweep::kLanes);
+        }
+    }
+    __device__ void finish(const Acc& a, const Self&, int i, const GcParams&) const {
+        count[i] = a.cnt;
+        hash[i] = a.h;
+    }
+};
 
 }  // namespace
 
@@ -347,12 +391,10 @@ int gc_cupar_AppFluidPeriodicBC(int n, int* d_sortpart, float* d_totalcoor, int*
 int gc_cupar_CalFluidDen(int n, float* d_totalcoor, float* d_velrhop, int* d_cc, int* d_ncube, float* d_outerregion,
                          int* d_sortpart, int* d_beginendcube) {
     if (gc_state().in_fused_step) return GC_OK;
-    (void)d_ncube; (void)d_outerregion;
+    (void)d_cc; (void)d_ncube; (void)d_outerregion;
     GC_PRE("CalFluidDen", true);
-    k_density<<<nb, SDPDSIZE, 0, s.stream>>>(n, p, (const float3*)d_totalcoor, (float4*)d_velrhop, (const int3*)d_cc,
-                                            d_sortpart, (const int2*)d_beginendcube);
-    GC_CHECK_LAUNCH("CalFluidDen");
-    return GC_OK;
+    return launch_sweep(DensityOp{(float4*)d_velrhop}, n, p, d_totalcoor, d_sortpart, d_beginendcube, s.stream,
+                        "CalFluidDen");
 }
 
 int gc_cupar_PredictFluidVel(int n, int* d_sortpart, float* d_velrhop, float* d_velhalf, float* d_totalforce) {
@@ -369,7 +411,7 @@ int gc_cupar_PredictFluidVel(int n, int* d_sortpart, float* d_velrhop, float* d_
 int gc_cupar_CalBound2Vel(int n, float* d_totalcoor, float* d_velrhop, int* d_cc, int* d_ncube, float* d_outerregion,
                           int* d_sortpart, int* d_beginendcube) {
     if (gc_state().in_fused_step) return GC_OK;
-    (void)d_ncube; (void)d_outerregion;
+    (void)d_cc; (void)d_ncube; (void)d_outerregion;
     GC_PRE("CalBound2Vel", true);
     if (p.nF == p.nB2) return GC_OK;   // no Bound2 particles
     // The prescribed wall velocity lives in the wall's VelHalf, which the
@@ -378,11 +420,8 @@ int gc_cupar_CalBound2Vel(int n, float* d_totalcoor, float* d_velrhop, int* d_cc
     // the latest PredictFluidVel / CorrectFliudVel (both precede every
     // CalBound2Vel in src/Particle.cu:1316-1327); without one the walls are
     // at rest.
-    k_bound2vel<<<nb, SDPDSIZE, 0, s.stream>>>(n, p, (const float3*)d_totalcoor, (float4*)d_velrhop,
-                                              (const float3*)s.velhalf_ptr, (const int3*)d_cc, d_sortpart,
-                                              (const int2*)d_beginendcube);
-    GC_CHECK_LAUNCH("CalBound2Vel");
-    return GC_OK;
+    return launch_sweep(Bound2VelOp{(float4*)d_velrhop, (const float3*)s.velhalf_ptr}, n, p, d_totalcoor, d_sortpart,
+                        d_beginendcube, s.stream, "CalBound2Vel");
 }
 
 int gc_cupar_EOS(int n, int* d_sortpart, float* d_velrhop, float* d_press) {
@@ -398,25 +437,25 @@ int gc_cupar_CalFluidSDPDForce(int n, float* h_sdpdforce, float* d_totalcoor, fl
                                int* d_ncube, int* d_sortpart, float* d_outerregion, int* d_beginendcube,
                                float* d_totalforce, float* d_press) {
     if (gc_state().in_fused_step) return GC_OK;
-    (void)h_sdpdforce; (void)d_ncube; (void)d_outerregion;
+    (void)h_sdpdforce; (void)d_cc; (void)d_ncube; (void)d_outerregion;
     GC_PRE("CalFluidSDPDForce", true);
-    k_sdpd<<<nb, SDPDSIZE, 0, s.stream>>>(n, p, (const float3*)d_totalcoor, (const float4*)d_velrhop,
-                                         (const int3*)d_cc, d_sortpart, (const int2*)d_beginendcube,
-                                         (float3*)d_totalforce, d_press);
-    GC_CHECK_LAUNCH("CalFluidSDPDForce");
-    return GC_OK;
+    const float4* vr = (const float4*)d_velrhop;
+    float3* fo = (float3*)d_totalforce;
+    if (p.noise_pref > 0.f)
+        return launch_sweep(SdpdOp<true>{vr, d_press, fo}, n, p, d_totalcoor, d_sortpart, d_beginendcube, s.stream,
+                            "CalFluidSDPDForce");
+    return launch_sweep(SdpdOp<false>{vr, d_press, fo}, n, p, d_totalcoor, d_sortpart, d_beginendcube, s.stream,
+                        "CalFluidSDPDForce");
 }
 
 int gc_cupar_CalFluidRepForce(int n, float* d_totalcoor, int* d_cc, int* d_ncube, int* d_sortpart,
                               float* d_outerregion, int* d_beginendcube, float* d_totalforce) {
     if (gc_state().in_fused_step) return GC_OK;
-    (void)d_ncube; (void)d_outerregion;
+    (void)d_cc; (void)d_ncube; (void)d_outerregion;
     GC_PRE("CalFluidRepForce", true);
     if (p.nB2 == 0) return GC_OK;   // no Bound1 particles
-    k_repulsion<<<nb, SDPDSIZE, 0, s.stream>>>(n, p, (const float3*)d_totalcoor, (const int3*)d_cc, d_sortpart,
-                                              (const int2*)d_beginendcube, (float3*)d_totalforce);
-    GC_CHECK_LAUNCH("CalFluidRepForce");
-    return GC_OK;
+    return launch_sweep(RepulsionOp{(float3*)d_totalforce}, n, p, d_totalcoor, d_sortpart, d_beginendcube, s.stream,
+                        "CalFluidRepForce");
 }
 
 int gc_cupar_SetFluidExtForce(int driveon, int n, int* d_sortpart, float* d_totalforce) {
@@ -444,10 +483,8 @@ int gc_cupar_CorrectFliudVel(int n, int* d_sortpart, float* d_totalforce, float*
 int gc_debug_neighbor_stats(int n, float* d_totalcoor, int* d_sortpart, int* d_beginendcube, int* d_count,
                             unsigned long long* d_hash) {
     GC_PRE("debug_neighbor_stats", true);
-    k_nbstats<<<nb, SDPDSIZE, 0, s.stream>>>(n, p, (const float3*)d_totalcoor, d_sortpart,
-                                            (const int2*)d_beginendcube, d_count, d_hash);
-    GC_CHECK_LAUNCH("debug_neighbor_stats");
-    return GC_OK;
+    return launch_sweep(NeighborOp{d_count, d_hash}, n, p, d_totalcoor, d_sortpart, d_beginendcube, s.stream,
+                        "debug_neighbor_stats");
 }
 
 }  // extern "C"

@@ -1,0 +1,331 @@
+// sweep.cuh -- the neighbour sweep of the boundary entry points that need the
+// pairs of a cube grid (density, SDPD force, wall repulsion, wall velocity).
+//
+// One block takes one cube at a time: all particles of a cube share the same
+// 27 cubes of candidates (about 760 at 27 particles per rc^3), which are
+// staged once in shared memory.  Eight lanes take two particles: they first
+// only mark the candidates within the cut-off (a bit each; one shared-memory
+// load serves both particles), then four lanes each evaluate the marked
+// candidates of one of the two in even shares.  About 15 % of the candidates
+// are partners: with one thread per particle testing and evaluating in one
+// loop, nearly every iteration ran the pair physics for one or two lanes of
+// a warp (17.5 of 32 lanes active, 4240 warp instructions per particle in
+// the SDPD sweep).  The lanes also give a small system enough warps: an 83
+// thousand particle channel is 650 blocks of one thread per particle, each a
+// serial chain of 750 candidates.
+//
+// Bound by instruction issue (80 % of the slots in the density sweep, 70 % in
+// the SDPD sweep, where shared memory holds six blocks a SM).  Measured on
+// one GB300: a million-particle suspension's step 6.73 -> 2.96 ms (density
+// 0.66 ms, SDPD 1.32 ms, the two together 5.7 ms before), an 83 thousand
+// particle channel with walls of both kinds 1.55 -> 0.43 ms.  One particle
+// per four lanes testing for itself took 0.86 and 1.51 ms (a shared-memory
+// load per test), without even shares 0.99 and 2.26 ms.
+//
+// Candidates are taken in the order of the cubes (z, y, x) and of their
+// slots, and the partial sums of the lanes are added by a fixed tree, so
+// results repeat bit for bit.
+#pragma once
+
+#include "gc_internal.cuh"
+
+#include <type_traits>
+
+namespace gcsweep {
+
+constexpr int kBlock = 128;              // threads per block
+constexpr int kGroup = 8;                // lanes that test candidates together, for two particles
+constexpr int kLanes = 4;                // lanes that evaluate a particle's partners
+constexpr int kPart = kBlock / kLanes;   // particles of a cube taken together
+constexpr int kCap = 896;                // candidates staged together
+constexpr int kWord = 32 * kGroup;       // candidates of one word of every lane's marks
+constexpr int kWords = (kCap + kWord - 1) / kWord;
+constexpr float kFar = 3.0e38f;          // coordinate of a candidate that takes no part (its r^2 is infinite)
+
+// Cubes a block takes one after the other: one where cubes hold eight
+// particles or more on average (a fluid has 27), more in a sparse grid, so
+// that a block has about eight particles to work on and the empty cubes do
+// not each cost a block.
+inline int cubes_per_block(long long n, long long K) {
+    long long c = n > 0 ? (8 * K + n - 1) / n : 1;
+    return c < 1 ? 1 : (c > 128 ? 128 : (int)c);
+}
+
+struct Shared {
+    float4 x[kCap];                      // position, id bits
+    unsigned mark[2][kWords * kBlock];   // per particle of the group: word w of thread t at w * kBlock + t
+    int beg[27], off[28];                // first slot of each cube of the stencil, their scanned sizes
+    float3 shift[27];                    // what brings each cube next to the centre
+};
+
+// First slots, scanned sizes (sh.off[27] is the number of candidates) and
+// shifts of the 27 cubes around cube c.  Cubes beyond a wall axis are empty;
+// periodic axes have at least three cubes, so none is taken twice.  A
+// stencil that crosses a periodic face is brought together below the lower
+// face: what lies at the upper face moves down by the box length, which is
+// exact in FP32 where the minimum image of the difference is not.
+__device__ __forceinline__ void stencil(const GcGrid& g, int3 c, const int2* __restrict__ bec, Shared& sh) {
+    if (threadIdx.x < 32) {
+        const int t = threadIdx.x;
+        int cnt = 0, b = 0;
+        if (t < 27) {
+            const int z = cube_step(c.z, t / 9 - 1, 2, g), y = cube_step(c.y, t / 3 % 3 - 1, 1, g),
+                      x = cube_step(c.x, t % 3 - 1, 0, g);
+            if (x >= 0 && y >= 0 && z >= 0) {
+                const int2 be = bec[cube_key(x, y, z, g)];
+                b = be.x;
+                cnt = max(be.y - be.x, 0);
+            }
+            auto down = [&](int cc, int q, int a) {
+                if (!(g.pmask & (1 << a))) return 0.f;
+                const int last = g.n[a] - 1;
+                return (cc == 0 && q == last) || (cc == last && q != 0) ? -g.L[a] : 0.f;
+            };
+            sh.shift[t] = f3(down(c.x, x, 0), down(c.y, y, 1), down(c.z, z, 2));
+        }
+        int sum = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (t >= o) sum += v;
+        }
+        if (t < 27) {
+            sh.beg[t] = b;
+            sh.off[t + 1] = sum;
+        }
+        if (t == 0) sh.off[0] = 0;
+    }
+    __syncthreads();
+}
+
+// Whether x lies outside the box on a periodic axis, or is no number.
+__device__ __forceinline__ bool outside(float3 x, const GcGrid& g) {
+    bool o = !(x.x == x.x && x.y == x.y && x.z == x.z);
+    if (g.pmask & 1) o |= !(x.x >= g.lo[0] && x.x < g.hi[0]);
+    if (g.pmask & 2) o |= !(x.y >= g.lo[1] && x.y < g.hi[1]);
+    if (g.pmask & 4) o |= !(x.z >= g.lo[2] && x.z < g.hi[2]);
+    return o;
+}
+
+template <bool IMAGE>
+__device__ __forceinline__ float3 diff(float3 a, float4 b, const GcGrid& g) {
+    if constexpr (IMAGE) return min_image(a, f3(b.x, b.y, b.z), g);
+    else return f3(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z));
+}
+
+// Marks the staged candidates [0, m) (m a multiple of 4 kGroup, padded with
+// far ones) within cut2 of xa and of xb that lane s tests; returns their
+// numbers (xa's in the low half).  Bit 31 - u of word w is the candidate
+// w * kWord + u * kGroup + s.
+//
+// The plain form takes seven instructions a candidate and particle: r^2 -
+// cut2 by fused multiply-adds and its sign shifted into the word (a pair
+// within a rounding of the cut-off, where every pair function here is zero,
+// may count or not).  With IMAGE the squared distance of the minimum image is
+// tested as the oracle tests it; a NaN distance counts as within, so that a
+// lost particle shows in its neighbours.
+template <bool IMAGE>
+__device__ __forceinline__ int mark(Shared& sh, float3 xa, float3 xb, int s, int m, float cut2, const GcGrid& g) {
+    int count = 0;
+    for (int w = 0, q0 = 0; q0 < m; ++w, q0 += kWord) {
+        const int it = min(32, (m - q0) / kGroup);
+        const float4* x = sh.x + q0 + s;
+        unsigned a = 0, b = 0;
+        for (int u0 = 0; u0 < it; u0 += 4) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float4 xj = x[(u0 + u) * kGroup];
+                const float3 da = diff<IMAGE>(xa, xj, g), db = diff<IMAGE>(xb, xj, g);
+                if constexpr (IMAGE) {
+                    a = (a << 1) | (norm2_rn(da) >= cut2 ? 0u : 1u);
+                    b = (b << 1) | (norm2_rn(db) >= cut2 ? 0u : 1u);
+                } else {
+                    const float ta = fmaf(da.x, da.x, fmaf(da.y, da.y, fmaf(da.z, da.z, -cut2)));
+                    const float tb = fmaf(db.x, db.x, fmaf(db.y, db.y, fmaf(db.z, db.z, -cut2)));
+                    a = __funnelshift_l(__float_as_uint(ta), a, 1);
+                    b = __funnelshift_l(__float_as_uint(tb), b, 1);
+                }
+            }
+        }
+        a <<= 32 - it;
+        b <<= 32 - it;
+        sh.mark[0][w * kBlock + threadIdx.x] = a;
+        sh.mark[1][w * kBlock + threadIdx.x] = b;
+        count += __popc(a) + (__popc(b) << 16);
+    }
+    return count;
+}
+
+// Evaluates op.pair(acc, ...) for an even share of the marked candidates of
+// this thread's particle (particle h of the group): lane s of its four takes
+// the ranks total s / 4 to total (s + 1) / 4 of the marks in the order of
+// lanes, words and bits.  (The marks found by four lanes differ by a third,
+// and the largest of a warp's shares sets its time.)  `count` as mark()
+// returned it.  Called by whole warps.
+template <bool IMAGE, class Op>
+__device__ __forceinline__ void evaluate(const Op& op, const typename Op::Extra& ex, const typename Op::Self& self,
+                                         typename Op::Acc& acc, const Shared& sh, float3 xi, int m, int count,
+                                         const GcParams& p) {
+    const int t = threadIdx.x % kGroup, h = t / kLanes, s = t % kLanes;
+    int end = count;   // inclusive scan over the group's lanes
+#pragma unroll
+    for (int o = 1; o < kGroup; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, end, o, kGroup);
+        if (t >= o) end += v;
+    }
+    auto of = [&](int v) { return (v >> (16 * h)) & 0xffff; };
+    const int total = of(__shfl_sync(0xffffffffu, end, kGroup - 1, kGroup));
+    int r = total * s / kLanes, n = total * (s + 1) / kLanes - r;
+    int lane = 0, base = 0;   // the lane whose marks hold rank r, and the marks before it
+#pragma unroll
+    for (int l = 0; l + 1 < kGroup; ++l) {
+        const int e = of(__shfl_sync(0xffffffffu, end, l, kGroup));
+        if (e <= r) {
+            lane = l + 1;
+            base = e;
+        }
+    }
+    if (n <= 0) return;
+    const unsigned* col = sh.mark[h] + (threadIdx.x & ~(kGroup - 1));
+    int w = 0;
+    unsigned bits = col[lane];
+    r -= base;
+    for (int c = __popc(bits); r >= c; c = __popc(bits)) {   // the word
+        r -= c;
+        bits = col[++w * kBlock + lane];
+    }
+    for (; r > 0; --r) bits &= ~(0x80000000u >> __clz(bits));   // the bit
+    const int words = (m + kWord - 1) / kWord;
+    for (; n > 0; --n) {
+        while (!bits) {   // ends: n marks are left
+            if (++w == words) {
+                w = 0;
+                ++lane;
+            }
+            bits = col[w * kBlock + lane];
+        }
+        const int u = __clz(bits);
+        bits &= ~(0x80000000u >> u);
+        const int q = w * kWord + u * kGroup + lane;
+        const float4 xj = sh.x[q];
+        const float3 d = diff<IMAGE>(xi, xj, p.g);
+        op.pair(acc, self, ex, q, __float_as_uint(xj.w), d, IMAGE ? norm2_rn(d) : norm2_fma(d), p);
+    }
+}
+
+// The sweep.  Op says which particles it is for (active), which candidates
+// take part (keep), what else of a candidate is staged (Extra, stage), the
+// cut-off, the pair function, what to do with the sum (finish) and with a
+// particle that it is not for (idle); with Op::kExact the neighbour predicate
+// is the oracle's, bit for bit.
+//
+// Positions are staged with the shift of their cube, and with every staged
+// position inside the box the plain difference of shifted positions is the
+// minimum image of every pair within a cube width (other pairs are beyond
+// the cut-off either way).  Where a staged position lies outside the box
+// (a caller that has not wrapped it), the unshifted positions are staged and
+// the image is formed pair by pair.
+template <class Op>
+__global__ void __launch_bounds__(kBlock, Op::kBlocks) k_sweep(int K, int per_block, GcParams p, Op op,
+                                                  const float3* __restrict__ coor, const int* __restrict__ sortpart,
+                                                  const int2* __restrict__ bec) {
+    __shared__ Shared sh;
+    __shared__ typename Op::Extra ex;
+    const GcGrid& g = p.g;
+    const int grp = threadIdx.x / kGroup, t = threadIdx.x % kGroup, h = t / kLanes;
+    const int k1 = min(K, (int)(blockIdx.x + 1) * per_block);
+    for (int cube = blockIdx.x * per_block; cube < k1; ++cube) {
+        const int2 be = bec[cube];
+        if (be.y <= be.x) continue;
+        bool any = false, own_out = false;
+        for (int i = be.x + threadIdx.x; i < be.y; i += kBlock) {
+            const unsigned id = (unsigned)sortpart[i];
+            if (op.active(id, p)) {
+                any = true;
+                own_out |= outside(coor[i], g);
+            } else {
+                op.idle(i);
+            }
+        }
+        if (!__syncthreads_or(any)) continue;
+        stencil(g, make_int3(cube % g.n[0], cube / g.n[0] % g.n[1], cube / g.n[0] / g.n[1]), bec, sh);
+        const int total = sh.off[27];
+        bool image = Op::kExact, some = false;
+        // stages the candidates [q0, q0 + cnt), padded with far ones to m
+        auto stage = [&](int q0, int cnt, int m, bool shifted, bool& out) {
+            bool kept = false;
+            for (int r = threadIdx.x / 32; r < 27; r += kBlock / 32) {
+                const int o = sh.off[r] - q0, e = min(sh.off[r + 1] - q0, cnt), j0 = sh.beg[r] - o;
+                const float3 v = sh.shift[r];
+                for (int q = max(o, 0) + (int)threadIdx.x % 32; q < e; q += 32) {
+                    const int j = j0 + q;
+                    const unsigned idj = (unsigned)sortpart[j];
+                    float4 x = make_float4(kFar, kFar, kFar, 0.f);
+                    if (op.keep(idj, p)) {
+                        const float3 y = coor[j];
+                        out |= outside(y, g);
+                        x = shifted ? make_float4(y.x + v.x, y.y + v.y, y.z + v.z, __uint_as_float(idj))
+                                    : make_float4(y.x, y.y, y.z, __uint_as_float(idj));
+                        kept = true;
+                        op.stage(ex, q, j, p);
+                    }
+                    sh.x[q] = x;
+                }
+            }
+            for (int q = cnt + threadIdx.x; q < m; q += kBlock) sh.x[q] = make_float4(kFar, kFar, kFar, 0.f);
+            return kept;
+        };
+        for (int b0 = be.x; b0 < be.y; b0 += kPart) {
+            // the group's two particles, and the one of them this thread evaluates
+            const int ia = b0 + 2 * grp, i = ia + h;
+            const unsigned id = i < be.y ? (unsigned)sortpart[i] : 0u;
+            const bool act = i < be.y && op.active(id, p);
+            const float3 own = act ? coor[i] : f3(-kFar, -kFar, -kFar);
+            typename Op::Acc acc;
+            typename Op::Self self;
+            op.begin(acc, self, i, id, act, p);
+            for (int q0 = 0; q0 < total; q0 += kCap) {
+                const int cnt = min(kCap, total - q0);
+                const int m = (cnt + 4 * kGroup - 1) / (4 * kGroup) * (4 * kGroup);
+                if (b0 == be.x || total > kCap) {   // the candidates stay staged for the cube's next particles
+                    __syncthreads();
+                    bool out = own_out;
+                    const bool kept = stage(q0, cnt, m, !Op::kExact, out);
+                    some = __syncthreads_or(kept);
+                    if (!Op::kExact) {
+                        image = __syncthreads_or(out);
+                        if (image) {
+                            stage(q0, cnt, m, false, out);
+                            __syncthreads();
+                        }
+                    }
+                }
+                if (!some || !__any_sync(0xffffffffu, act)) continue;
+                auto both = [&](auto im) {
+                    constexpr bool I = decltype(im)::value;
+                    const float3 v = I ? f3(0.f, 0.f, 0.f) : sh.shift[13];
+                    const float3 xi = f3(own.x + v.x, own.y + v.y, own.z + v.z);
+                    const float3 xo = f3(__shfl_xor_sync(0xffffffffu, xi.x, kLanes), __shfl_xor_sync(0xffffffffu, xi.y, kLanes),
+                                         __shfl_xor_sync(0xffffffffu, xi.z, kLanes));
+                    const int count = mark<I>(sh, h ? xo : xi, h ? xi : xo, t, m, op.cut2(p), g);
+                    __syncwarp();
+                    evaluate<I>(op, ex, self, acc, sh, xi, m, count, p);
+                };
+                if (image) both(std::true_type{});
+                else both(std::false_type{});
+                __syncwarp();   // the marks are written again for the next candidates
+            }
+            op.reduce(acc);
+            if (act && t % kLanes == 0) op.finish(acc, self, i, p);
+        }
+    }
+}
+
+// Adds v over the lanes of a particle (a fixed tree).
+__device__ __forceinline__ float lane_sum(float v) {
+#pragma unroll
+    for (int o = kLanes / 2; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, kLanes);
+    return v;
+}
+
+}  // namespace gcsweep

@@ -102,3 +102,41 @@ def test_unwrapped_positions(cuda_device, kind):
     np.testing.assert_allclose(b["rho"][fluid], a["rho"][fluid], rtol=2 * 100 * U)
     scale = np.abs(a["press"]).max() / a["rho"].min() ** 2 * 67.0 * 100
     np.testing.assert_allclose(b["force"], a["force"], rtol=0, atol=scale * 2 * 100 * U * 20)
+
+
+@pytest.mark.parametrize("ncells,subdiv", [(1, 2), (7, 1), (40, 2)])
+def test_aggregation_matches_oracle(cuda_device, ncells, subdiv):
+    """From one cell (no pair) to forty interpenetrating ones in a box of
+    seven cubes: more vertices in a cube and in a stencil than a block takes
+    at once, stencils across every periodic face."""
+    from gpucell_gb300.host import ParticleSystem
+    from oracle.binding import Oracle, assert_forces_close
+    phys = gen.Physics(ext_force=0.0, sur_energy=3.0e-3, sca_fac=1.5, zero_len=0.3, max_cut=2.5)
+    rng = np.random.default_rng(ncells)
+    L = 7.25
+    verts, faces = gen.icosphere(subdiv)
+    shape = gen.biconcave(verts, 3.0)
+    cells = [(shape @ gen.random_rotation(rng).T + rng.uniform(0, L, 3) * 0.999, faces) for _ in range(ncells)]
+    fluid = rng.uniform(0, L, (2000, 3))
+    none = np.zeros((0, 3))
+    cfg = gen._assemble("packed", [0, L, 0, L, 0, L], 7, none, none, fluid, cells, phys, 1.0 / 3.0)
+    ps, o = ParticleSystem(cfg, noise=False), Oracle(cfg, noise=False)
+    o.setup()
+    wrapped = np.mod(cfg.coor, np.float32(L)).astype(np.float32)
+    o.set(pos=wrapped)
+    ps.set_state(pos=wrapped)
+    ps.con_cube_list()
+    area = ps.d["ParArea"].cpu().numpy()
+    o.set(pararea=area)
+    z = np.zeros((cfg.n, 3))
+    ps.set_state(force=z)
+    o.set(force=z)
+    ps.agg_force()
+    o.call("agg_force")
+    g = ps.fetch()
+    s = o.force_scale(o.SCALE_MORSE)
+    # e^{beta (r0 - r)} of a rounded argument up to 3.3, squared, and the sum over the lanes
+    k = 64 + cfg.ncp / 8
+    assert_forces_close(g["force"], o.force, s, k=k, what="aggregation")
+    assert_forces_close(g["AggForce"], o.aggforce, s[cfg.n_cell_start:], k=k, what="aggregation per vertex")
+    assert ncells == 1 or np.abs(o.aggforce).max() > 0

@@ -378,18 +378,116 @@ __global__ void __launch_bounds__(kMaxBS, GC_BUILD_MIN_BLOCKS) fk_build_list(int
 // and the number of set bits in ccnt.  The force pass then iterates only the
 // set bits, so no lane idles on an entry that does not act.
 
+// Lanes per particle of the list passes.  One thread per particle fills the
+// GPU from a few hundred thousand particles on; a smaller system then is a
+// serial chain of ~110 gathers per thread on a few warps per SM (134 us of
+// force pass for 6 thousand particles as for 80 thousand), so it takes its
+// entries with several lanes per particle, whose partial sums are added by a
+// fixed tree.
+constexpr int kWallLanes = 8;   // lanes per Bound2 particle
+
+// Lanes of a particle's group within its warp.
+template <int L>
+__device__ __forceinline__ unsigned group_mask() {
+    return (L >= 32 ? 0xffffffffu : (1u << (L & 31)) - 1u) << ((threadIdx.x & 31) & ~(L - 1));
+}
+
+template <int L>
+__device__ __forceinline__ float group_sum(float v, unsigned mask) {
+#pragma unroll
+    for (int o = L / 2; o; o >>= 1) v += __shfl_xor_sync(mask, v, o, L);
+    return v;
+}
+
+// K10 -- no-slip velocity of the Bound2 particle with wall index q / kWallLanes
+// (the Bound2 ids of all systems in order) from its list of moving
+// neighbours, reading and writing v.  Eight lanes per wall particle, four
+// entries in flight each: one thread per wall particle is a chain of 60
+// dependent gathers that set the length of its pass (54 us of a 190 us step
+// of a 6 thousand particle channel, 71 us at 350 thousand).
+template <bool ENS>
+__device__ __forceinline__ void wall_velocity(int q, int nwall, int n, const GcParams& p, const SysInfo& s0,
+                                              const SysInfo* __restrict__ sys, int nsys,
+                                              const int* __restrict__ slot_of, const float4* __restrict__ pos,
+                                              float4* __restrict__ v, const float4* __restrict__ vh,
+                                              const int* __restrict__ nbr, const int* __restrict__ cnt, int cap) {
+    const int w = q / kWallLanes, s = q % kWallLanes;
+    if (w >= nwall) return;   // whole groups
+    int k0 = 0;
+    if (ENS) {   // the system that holds wall particle w
+        int hi = nsys - 1;
+        while (k0 < hi) {
+            const int mid = (k0 + hi + 1) >> 1;
+            if ((int)sys[mid].w0 <= w) k0 = mid;
+            else hi = mid - 1;
+        }
+    }
+    const SysInfo& S = ENS ? sys[k0] : s0;
+    const int i = slot_of[S.b2 + (unsigned)(w - (int)S.w0)];
+    const Box B = box_of(S);
+    const float3 xi = xyz(pos[i]);
+    const int c = cnt[i];
+    const int* lp = nbr + sell(i, 0, cap);
+    float3 num = f3(0.f, 0.f, 0.f);
+    float den = 0.f;
+    constexpr int U = 4;
+    for (int k = s; k < c; k += U * kWallLanes) {
+        int j[U];
+        float r2[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) j[u] = k + u * kWallLanes < c ? __ldg(lp + (size_t)(k + u * kWallLanes) * 32) : n;
+#pragma unroll
+        for (int u = 0; u < U; ++u) r2[u] = norm2_rn(pair_image(xi, xyz(pos[j[u]]), B));
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (j[u] == n || r2[u] >= p.rc2) continue;
+            const float wt = wendland_w(r2[u] > 0.f ? r2[u] * rsqrtf(r2[u]) : 0.f, p);
+            const float4 vj = v[j[u]];
+            num += wt * f3(vj.x, vj.y, vj.z);
+            den += wt;
+        }
+    }
+    const unsigned gm = group_mask<kWallLanes>();
+    num = f3(group_sum<kWallLanes>(num.x, gm), group_sum<kWallLanes>(num.y, gm), group_sum<kWallLanes>(num.z, gm));
+    den = group_sum<kWallLanes>(den, gm);
+    if (s != 0) return;
+    const float4 w4 = vh[i];
+    const float3 r = den > 0.f ? f3(2.f * w4.x - num.x / den, 2.f * w4.y - num.y / den, 2.f * w4.z - num.z / den)
+                               : f3(w4.x, w4.y, w4.z);
+    v[i] = make_float4(r.x, r.y, r.z, 0.f);
+}
+
+template <bool ENS>
+__global__ void fk_wallvel(int nwall, int n, GcParams p, SysInfo s0, const SysInfo* __restrict__ sys, int nsys,
+                           const int* __restrict__ slot_of, const float4* __restrict__ pos, float4* __restrict__ v,
+                           const float4* __restrict__ vh, const int* __restrict__ nbr, const int* __restrict__ cnt,
+                           int cap) {
+    wall_velocity<ENS>(blockIdx.x * blockDim.x + threadIdx.x, nwall, n, p, s0, sys, nsys, slot_of, pos, v, vh, nbr, cnt,
+                       cap);
+}
+
 #ifndef GC_DENS_MIN_BLOCKS
 #define GC_DENS_MIN_BLOCKS 5
 #endif
 
-template <bool ENS, bool B1>
+// The first `wall_blocks` blocks give the Bound2 particles their velocity
+// (first, as theirs are the longest chains), the others take L lanes per
+// particle.
+template <bool ENS, bool B1, int L>
 __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, GcParams p, SysInfo s0, const SysInfo* __restrict__ sys,
                                                   const int* __restrict__ sysid, const float4* __restrict__ pos,
                                                   float4* __restrict__ vpred, const float4* __restrict__ vh,
                                                   float2* __restrict__ dp, const int* __restrict__ nbr,
                                                   const int* __restrict__ cnt, int cap, unsigned* __restrict__ cmask,
-                                                  int mw, int* __restrict__ ccnt, float wrap_margin) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+                                                  int mw, int* __restrict__ ccnt, float wrap_margin, int wall_blocks,
+                                                  int nwall, int nsys, const int* __restrict__ slot_of) {
+    if ((int)blockIdx.x < wall_blocks) {
+        wall_velocity<ENS>(blockIdx.x * blockDim.x + threadIdx.x, nwall, n, p, s0, sys, nsys, slot_of, pos, vpred, vh,
+                           nbr, cnt, cap);
+        return;
+    }
+    const int q = (blockIdx.x - wall_blocks) * blockDim.x + threadIdx.x;
+    const int i = q / L, s = q % L;
     if (i >= n) return;
     float4 xi4 = pos[i];
     float3 xi = xyz(xi4);
@@ -398,95 +496,84 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
     const Box B = box_of(S);
     const unsigned b2 = S.b2;
     int t = stype(id, S);
-    int c = cnt[i];
-    const int* lp = nbr + sell(i, 0, cap);
-    if (t == PT_FLUID || t == PT_MEMB) {
-        // the sum of W / wnorm, the particle's own share (W(0) / wnorm = 1)
-        // first; wnorm multiplies it once at the end
-        float acc = 1.f;
-        const float inv_rc4 = 4.f * p.inv_rc;
-        int kc = 0;
-        // The list is padded to a multiple of four entries with the sentinel
-        // slot.  Entries go in groups of four: the indices of the next group
-        // are loaded while the current group is evaluated, so that a thread
-        // keeps four index loads and four position loads in flight; the
-        // acting-entry bits of each 32-entry word are stored once.  The
-        // lanes of a warp read each line of the list together, once: the
-        // index loads stream (evict first), so that the list does not push
-        // the particle data the gathers need out of the caches.
-        const int c4 = (c + 3) & ~3;
-        auto run = [&](auto wrap) {
-            constexpr bool W = decltype(wrap)::value;
-            int jq[4];
-            if (c4 > 0) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) jq[u] = __ldcs(lp + (size_t)u * 32);
-            }
-            for (int w0 = 0; w0 < c4; w0 += 32) {
-                unsigned m = 0;
-                const int wend = min(w0 + 32, c4);
-                for (int k0 = w0; k0 < wend; k0 += 4) {
-                    float4 xj[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) xj[u] = pos[jq[u]];
-                    if (k0 + 4 < c4) {
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) jq[u] = __ldcs(lp + (size_t)(k0 + 4 + u) * 32);
-                    }
-                    // without branches: W is formed for every entry and added
-                    // (as +0 when the entry does not count, which leaves the sum
-                    // as it is), so that no lane waits on another's branch
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float3 dd = pair_diff<W>(xi, xyz(xj[u]), B);
-                        const float r2 = norm2_fma(dd);
-                        // without Bound1 walls in any system (B1 false) every partner is SDPD
-                        const bool in = r2 < p.rc2, apart = r2 > 0.f, sdpd = !B1 || fid(xj[u]) >= b2;
-                        const float r = apart ? r2 * rsqrt_ftz(r2) : 0.f;
-                        // (1 - s)^4 (1 + 4 s), s = r / rc
-                        const float tt = fmaf(-r, p.inv_rc, 1.f), t2 = tt * tt;
-                        acc += in && sdpd ? t2 * t2 * fmaf(r, inv_rc4, 1.f) : 0.f;
-                        // acting: an SDPD partner within rc, or a Bound1 wall within the repulsion range
-                        const bool act = in && apart && (sdpd || (B1 && r2 < p.rep_r0sq));
-                        m |= (unsigned)act << (k0 - w0 + u);
-                    }
-                }
-                if (cmask) {
-                    cmask[mrow(i, w0 >> 5, mw)] = m;
-                    kc += __popc(m);
-                }
-            }
-        };
-        // one form per warp (the image where any of its particles is near a
-        // periodic face), so that a warp does not run both
-        if (__any_sync(__activemask(), near_face(xi, S.g, wrap_margin))) run(std::true_type{});
-        else run(std::false_type{});
-        if (ccnt) ccnt[i] = kc;
-        const float sum = p.wnorm * acc;
-        float rho = p.mass * sum;
-        float c2 = (t == PT_MEMB) ? p.c2sq : p.c1sq;
-        float inv_d = __frcp_rn(sum);
-        dp[i] = make_float2(inv_d, c2 * (rho - p.rho0) * inv_d * inv_d);
+    if (t != PT_FLUID && t != PT_MEMB) {
+        if (s == 0) dp[i] = make_float2(p.mass / p.rho0, 0.f);
         return;
     }
-    dp[i] = make_float2(p.mass / p.rho0, 0.f);
-    if (t != PT_B2) return;
-    float3 num = f3(0.f, 0.f, 0.f);
-    float den = 0.f;
-    for (int k = 0; k < c; ++k) {
-        int j = __ldg(lp + (size_t)k * 32);
-        float r2 = norm2_rn(pair_image(xi, xyz(pos[j]), B));
-        if (r2 >= p.rc2) continue;
-        float r = r2 > 0.f ? r2 * rsqrtf(r2) : 0.f;
-        float w = wendland_w(r, p);
-        float4 vj = vpred[j];
-        num += w * f3(vj.x, vj.y, vj.z);
-        den += w;
-    }
-    float4 w4 = vh[i];
-    float3 v = den > 0.f ? f3(2.f * w4.x - num.x / den, 2.f * w4.y - num.y / den, 2.f * w4.z - num.z / den)
-                         : f3(w4.x, w4.y, w4.z);
-    vpred[i] = make_float4(v.x, v.y, v.z, 0.f);
+    const unsigned gm = group_mask<L>();
+    int c = cnt[i];
+    const int* lp = nbr + sell(i, 0, cap);
+    // the sum of W / wnorm, the particle's own share (W(0) / wnorm = 1)
+    // first; wnorm multiplies it once at the end
+    float acc = s == 0 ? 1.f : 0.f;
+    const float inv_rc4 = 4.f * p.inv_rc;
+    int kc = 0;
+    // The list is padded to a multiple of four entries with the sentinel
+    // slot.  Entries go in groups of four: the indices of the next group
+    // are loaded while the current group is evaluated, so that a thread
+    // keeps four index loads and four position loads in flight; the
+    // acting-entry bits of each 32-entry word are stored once.  Lane s of L
+    // takes the groups s, s + L, ... of each word, and the lanes' bits are
+    // put together by shuffles.  The lanes of a warp read each line of the
+    // list together, once: the index loads stream (evict first), so that the
+    // list does not push the particle data the gathers need out of the caches.
+    const int c4 = (c + 3) & ~3;
+    auto run = [&](auto wrap) {
+        constexpr bool W = decltype(wrap)::value;
+        int jq[4];
+        if (4 * s < c4) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) jq[u] = __ldcs(lp + (size_t)(4 * s + u) * 32);
+        }
+        for (int w0 = 0; w0 < c4; w0 += 32) {
+            unsigned m = 0;
+            const int wend = min(w0 + 32, c4);
+            for (int k0 = w0 + 4 * s; k0 < wend; k0 += 4 * L) {
+                float4 xj[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) xj[u] = pos[jq[u]];
+                if (k0 + 4 * L < c4) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) jq[u] = __ldcs(lp + (size_t)(k0 + 4 * L + u) * 32);
+                }
+                // without branches: W is formed for every entry and added
+                // (as +0 when the entry does not count, which leaves the sum
+                // as it is), so that no lane waits on another's branch
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float3 dd = pair_diff<W>(xi, xyz(xj[u]), B);
+                    const float r2 = norm2_fma(dd);
+                    // without Bound1 walls in any system (B1 false) every partner is SDPD
+                    const bool in = r2 < p.rc2, apart = r2 > 0.f, sdpd = !B1 || fid(xj[u]) >= b2;
+                    const float r = apart ? r2 * rsqrt_ftz(r2) : 0.f;
+                    // (1 - s)^4 (1 + 4 s), s = r / rc
+                    const float tt = fmaf(-r, p.inv_rc, 1.f), t2 = tt * tt;
+                    acc += in && sdpd ? t2 * t2 * fmaf(r, inv_rc4, 1.f) : 0.f;
+                    // acting: an SDPD partner within rc, or a Bound1 wall within the repulsion range
+                    const bool act = in && apart && (sdpd || (B1 && r2 < p.rep_r0sq));
+                    m |= (unsigned)act << (k0 - w0 + u);
+                }
+            }
+            if (cmask) {
+#pragma unroll
+                for (int o = L / 2; o; o >>= 1) m |= __shfl_xor_sync(gm, m, o, L);
+                if (s == 0) cmask[mrow(i, w0 >> 5, mw)] = m;
+                kc += __popc(m);
+            }
+        }
+    };
+    // one form per warp (the image where any of its particles is near a
+    // periodic face), so that a warp does not run both
+    if (__any_sync(__activemask(), near_face(xi, S.g, wrap_margin))) run(std::true_type{});
+    else run(std::false_type{});
+    acc = group_sum<L>(acc, gm);
+    if (s != 0) return;
+    if (ccnt) ccnt[i] = kc;
+    const float sum = p.wnorm * acc;
+    float rho = p.mass * sum;
+    float c2 = (t == PT_MEMB) ? p.c2sq : p.c1sq;
+    float inv_d = __frcp_rn(sum);
+    dp[i] = make_float2(inv_d, c2 * (rho - p.rho0) * inv_d * inv_d);
 }
 
 // ---------------------------------------------------------------------------
@@ -530,16 +617,19 @@ __global__ void fk_pack_vel(int n, const float4* __restrict__ v, uint2* __restri
     out[i] = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
 }
 
-template <bool COMPACT, bool ENS, bool HALFV, bool NOISE, bool B1>
-__global__ void __launch_bounds__(kMaxBS, force_min_blocks(ENS))
+// L lanes per particle take even shares of its entries (ranks c s / L to
+// c (s + 1) / L), in the order of the list.
+template <bool COMPACT, bool ENS, bool HALFV, bool NOISE, bool B1, int L>
+__global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
     fk_force(int n, GcParams p, SysInfo s0, const SysInfo* __restrict__ sys, const int* __restrict__ sysid,
              const unsigned* __restrict__ nkey, const float4* __restrict__ pos, const float4* __restrict__ vpred,
              const float4* __restrict__ vh, const float2* __restrict__ dp, float4* __restrict__ force,
              float4* __restrict__ vel, const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
              const unsigned* __restrict__ cmask, int mw, const float4* __restrict__ mforce, int drive,
              const uint2* __restrict__ vph, float wrap_margin) {
-    constexpr int G = kForceGroup;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int G = L > 1 ? 2 : kForceGroup;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = q / L, ln = q % L;
     if (i >= n) return;
     float4 xi4 = pos[i];
     float3 xi = xyz(xi4);
@@ -547,7 +637,7 @@ __global__ void __launch_bounds__(kMaxBS, force_min_blocks(ENS))
     const int s = ENS ? (sysid ? sysid[i] : 0) : 0;
     GC_SYS_OF(S, i);
     if (id < S.fl) {
-        force[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ln == 0) force[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
     const Box B = box_of(S);
@@ -559,11 +649,26 @@ __global__ void __launch_bounds__(kMaxBS, force_min_blocks(ENS))
     float4 vi = vpred[i];
     float2 dpi = dp[i];
     float3 f = f3(0.f, 0.f, 0.f);
-    int c = cnt[i];
+    const int call = cnt[i];
+    const int first = call * ln / L;                     // this lane's entries
+    const int c = call * (ln + 1) / L - first;
     const int* lp = nbr + sell(i, 0, cap);
     const unsigned* mp = COMPACT ? cmask + mrow(i, 0, mw) : nullptr;
     unsigned m = 0;
     int base = -32;
+    if constexpr (COMPACT && L > 1) {
+        // the mask word and bit of acting entry `first` (it exists where this lane has entries)
+        int r = first;
+        while (c > 0) {
+            base += 32;
+            m = __ldg(mp + (size_t)(base >> 5) * 32);
+            const int here = __popc(m);
+            if (r < here) break;
+            r -= here;
+        }
+        if (c > 0)
+            for (; r > 0; --r) m &= m - 1;
+    }
     // index of the next acting entry (COMPACT) or of the next entry; called
     // once per entry, in order.  The scan for a non-empty mask word ends: it
     // runs only while k < c, and c = ccnt[i] is the number of bits set in the
@@ -585,7 +690,7 @@ __global__ void __launch_bounds__(kMaxBS, force_min_blocks(ENS))
             m &= m - 1;
             return base + b;
         } else {
-            return k;
+            return first + k;
         }
     };
     constexpr int A = kForceAhead;
@@ -670,6 +775,11 @@ __global__ void __launch_bounds__(kMaxBS, force_min_blocks(ENS))
     // every listed pair there); any other warp forms the image.
     if (__any_sync(__activemask(), near_face(xi, S.g, wrap_margin))) run(std::true_type{});
     else run(std::false_type{});
+    if constexpr (L > 1) {
+        const unsigned gm = group_mask<L>();
+        f = f3(group_sum<L>(f.x, gm), group_sum<L>(f.y, gm), group_sum<L>(f.z, gm));
+        if (ln != 0) return;
+    }
     if (drive) f.x += S.gx;
     if (id >= S.cs && mforce) {
         float4 mf = mforce[S.m0 + (id - S.cs)];
@@ -681,37 +791,6 @@ __global__ void __launch_bounds__(kMaxBS, force_min_blocks(ENS))
     float4 h = vh[i];
     float sc = 0.5f * p.dt * p.inv_mass;
     vel[i] = make_float4(h.x + sc * f.x, h.y + sc * f.y, h.z + sc * f.z, 0.f);
-}
-
-// second K10: wall velocity from the corrected velocities
-template <bool ENS>
-__global__ void fk_wallvel(int n, GcParams p, SysInfo s0, const SysInfo* __restrict__ sys,
-                           const int* __restrict__ sysid, const float4* __restrict__ pos, float4* __restrict__ vel,
-                           const float4* __restrict__ vh, const int* __restrict__ nbr, const int* __restrict__ cnt,
-                           int cap) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 xi4 = pos[i];
-    GC_SYS_OF(S, i);
-    if (stype(fid(xi4), S) != PT_B2) return;
-    const Box B = box_of(S);
-    float3 xi = xyz(xi4);
-    float3 num = f3(0.f, 0.f, 0.f);
-    float den = 0.f;
-    int c = cnt[i];
-    for (int k = 0; k < c; ++k) {
-        int j = __ldg(nbr + sell(i, k, cap));
-        float r2 = norm2_rn(pair_image(xi, xyz(pos[j]), B));
-        if (r2 >= p.rc2) continue;
-        float w = wendland_w(r2 > 0.f ? r2 * rsqrtf(r2) : 0.f, p);
-        float4 vj = vel[j];
-        num += w * f3(vj.x, vj.y, vj.z);
-        den += w;
-    }
-    float4 w4 = vh[i];
-    float3 v = den > 0.f ? f3(2.f * w4.x - num.x / den, 2.f * w4.y - num.y / den, 2.f * w4.z - num.z / den)
-                         : f3(w4.x, w4.y, w4.z);
-    vel[i] = make_float4(v.x, v.y, v.z, 0.f);
 }
 
 // ---------------------------------------------------------------------------
@@ -1731,30 +1810,32 @@ int launch_integrate(GcFused* f, cudaStream_t st, const GcParams& p) {
     return GC_OK;
 }
 
+template <int L>
+void density_launch(GcFused* f, cudaStream_t st, const GcParams& p, unsigned* cm, int* cc) {
+    const int bs = f->block, wb = gc_blocks((long long)f->nwall * kWallLanes, bs);
+    const int nb = wb + gc_blocks((long long)f->n * L, bs);
+    auto go = [&](auto ens, auto b1) {
+        fk_density<decltype(ens)::value, decltype(b1)::value, L><<<nb, bs, 0, st>>>(
+            f->n, p, s0(f), f->dsys, f->a.sys, f->a.pos, f->a.vpred, f->a.vh, f->dp, f->nbr, f->cnt, f->cap, cm, f->mw,
+            cc, wrap_margin(f), wb, f->nwall, f->nsys, f->slot_of);
+    };
+    if (f->ens) {
+        if (f->has_b1) go(std::true_type{}, std::true_type{});
+        else go(std::true_type{}, std::false_type{});
+    } else {
+        if (f->has_b1) go(std::false_type{}, std::true_type{});
+        else go(std::false_type{}, std::false_type{});
+    }
+}
+
 int launch_density(GcFused* f, cudaStream_t st, const GcParams& p, bool mark) {
     if (!f->lists) return launch_tile_density(f, st, p, false);
-    const int n = f->n, nb = gc_blocks(n, f->block);
     unsigned* cm = mark && f->compact ? f->cmask : nullptr;
     int* cc = mark && f->compact ? f->ccnt : nullptr;
-    if (f->ens) {
-        if (f->has_b1)
-            fk_density<true, true><<<nb, f->block, 0, st>>>(n, p, s0(f), f->dsys, f->a.sys, f->a.pos, f->a.vpred,
-                                                            f->a.vh, f->dp, f->nbr, f->cnt, f->cap, cm, f->mw, cc,
-                                                            wrap_margin(f));
-        else
-            fk_density<true, false><<<nb, f->block, 0, st>>>(n, p, s0(f), f->dsys, f->a.sys, f->a.pos, f->a.vpred,
-                                                             f->a.vh, f->dp, f->nbr, f->cnt, f->cap, cm, f->mw, cc,
-                                                             wrap_margin(f));
-    } else {
-        if (f->has_b1)
-            fk_density<false, true><<<nb, f->block, 0, st>>>(n, p, s0(f), f->dsys, f->a.sys, f->a.pos, f->a.vpred,
-                                                             f->a.vh, f->dp, f->nbr, f->cnt, f->cap, cm, f->mw, cc,
-                                                             wrap_margin(f));
-        else
-            fk_density<false, false><<<nb, f->block, 0, st>>>(n, p, s0(f), f->dsys, f->a.sys, f->a.pos, f->a.vpred,
-                                                              f->a.vh, f->dp, f->nbr, f->cnt, f->cap, cm, f->mw, cc,
-                                                              wrap_margin(f));
-    }
+    if (f->lanes == 8) density_launch<8>(f, st, p, cm, cc);
+    else if (f->lanes == 4) density_launch<4>(f, st, p, cm, cc);
+    else if (f->lanes == 2) density_launch<2>(f, st, p, cm, cc);
+    else density_launch<1>(f, st, p, cm, cc);
     GC_CHECK_LAUNCH("fused: density");
     return GC_OK;
 }
@@ -1788,33 +1869,45 @@ int launch_membranes(GcFused* f, cudaStream_t st, const GcParams& p) {
     return GC_OK;
 }
 
-template <bool COMPACT, bool HALFV, bool NOISE, bool B1>
+template <bool COMPACT, bool HALFV, bool NOISE, bool B1, int L>
 void force_launch_n(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
-    const int n = f->n, nb = gc_blocks(n, f->block);
+    const int n = f->n, nb = gc_blocks((long long)n * L, f->block);
     const float4* mf = f->ncell > 0 ? f->mforce : nullptr;
     const int* c = COMPACT ? f->ccnt : f->cnt;
     const unsigned* cm = COMPACT ? f->cmask : nullptr;
     const unsigned* nk = f->ens || f->capturing ? f->nkey : nullptr;
     if (f->ens)
-        fk_force<COMPACT, true, HALFV, NOISE, B1><<<nb, f->block, 0, st>>>(
+        fk_force<COMPACT, true, HALFV, NOISE, B1, L><<<nb, f->block, 0, st>>>(
             n, p, s0(f), f->dsys, f->a.sys, nk, f->a.pos, f->a.vpred, f->a.vh, f->dp, f->a.force, f->a.vel,
             f->nbr, c, f->cap, cm, f->mw, mf, drive, f->vph, wrap_margin(f));
     else
-        fk_force<COMPACT, false, HALFV, NOISE, B1><<<nb, f->block, 0, st>>>(
+        fk_force<COMPACT, false, HALFV, NOISE, B1, L><<<nb, f->block, 0, st>>>(
             n, p, s0(f), f->dsys, f->a.sys, nk, f->a.pos, f->a.vpred, f->a.vh, f->dp, f->a.force, f->a.vel,
             f->nbr, c, f->cap, cm, f->mw, mf, drive, f->vph, wrap_margin(f));
 }
 
-template <bool COMPACT, bool HALFV>
-void force_launch(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
+template <bool COMPACT, bool HALFV, int L>
+void force_launch_l(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
     const bool noise = p.noise_pref > 0.f;
     if (f->has_b1) {
-        if (noise) force_launch_n<COMPACT, HALFV, true, true>(f, st, p, drive);
-        else force_launch_n<COMPACT, HALFV, false, true>(f, st, p, drive);
+        if (noise) force_launch_n<COMPACT, HALFV, true, true, L>(f, st, p, drive);
+        else force_launch_n<COMPACT, HALFV, false, true, L>(f, st, p, drive);
     } else {
-        if (noise) force_launch_n<COMPACT, HALFV, true, false>(f, st, p, drive);
-        else force_launch_n<COMPACT, HALFV, false, false>(f, st, p, drive);
+        if (noise) force_launch_n<COMPACT, HALFV, true, false, L>(f, st, p, drive);
+        else force_launch_n<COMPACT, HALFV, false, false, L>(f, st, p, drive);
     }
+}
+
+// Several lanes per particle where the handle has them, for the forms in
+// ordinary use (compacted entries, FP32 velocities).
+template <bool COMPACT, bool HALFV>
+void force_launch(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
+    if constexpr (COMPACT && !HALFV) {
+        if (f->lanes == 8) return force_launch_l<true, false, 8>(f, st, p, drive);
+        if (f->lanes == 4) return force_launch_l<true, false, 4>(f, st, p, drive);
+        if (f->lanes == 2) return force_launch_l<true, false, 2>(f, st, p, drive);
+    }
+    force_launch_l<COMPACT, HALFV, 1>(f, st, p, drive);
 }
 
 int launch_force(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
@@ -1838,15 +1931,17 @@ bool any_bound2(const GcFused* f) {
     return false;
 }
 
-int launch_wallvel(GcFused* f, cudaStream_t st, const GcParams& p) {
-    if (!any_bound2(f)) return GC_OK;
-    const int n = f->n, nb = gc_blocks(n, f->block);
+// K10 on its own: the wall velocities in v from the moving particles' there
+// (after the corrector; and for the pair tiles, after their density pass).
+int launch_walls(GcFused* f, cudaStream_t st, const GcParams& p, float4* v) {
+    if (f->nwall == 0) return GC_OK;
+    const int nb = gc_blocks((long long)f->nwall * kWallLanes, f->block);
     if (f->ens)
-        fk_wallvel<true><<<nb, f->block, 0, st>>>(n, p, s0(f), f->dsys, f->a.sys, f->a.pos, f->a.vel, f->a.vh, f->nbr,
-                                                   f->cnt, f->cap);
+        fk_wallvel<true><<<nb, f->block, 0, st>>>(f->nwall, f->n, p, s0(f), f->dsys, f->nsys, f->slot_of, f->a.pos, v,
+                                                  f->a.vh, f->nbr, f->cnt, f->cap);
     else
-        fk_wallvel<false><<<nb, f->block, 0, st>>>(n, p, s0(f), f->dsys, f->a.sys, f->a.pos, f->a.vel, f->a.vh,
-                                                    f->nbr, f->cnt, f->cap);
+        fk_wallvel<false><<<nb, f->block, 0, st>>>(f->nwall, f->n, p, s0(f), f->dsys, f->nsys, f->slot_of, f->a.pos, v,
+                                                   f->a.vh, f->nbr, f->cnt, f->cap);
     GC_CHECK_LAUNCH("fused: wall velocity");
     return GC_OK;
 }
@@ -1901,7 +1996,7 @@ int one_step(GcFused* f, int drive) {
     prof_mark(f, st);
     GC_TRY(launch_force(f, st, p, drive));
     prof_mark(f, st);
-    GC_TRY(launch_wallvel(f, st, p));
+    GC_TRY(launch_walls(f, st, p, f->a.vel));
     if (f->early) GC_TRY(f->early(f, st, 3));
     f->steps++;
     return GC_OK;
@@ -1988,7 +2083,7 @@ int capture_step(GcFused* f, int drive) {
         if ((rc = launch_density(f, st, p, true)) != GC_OK) break;
         if ((rc = join_membranes(f, st)) != GC_OK) break;
         if ((rc = launch_force(f, st, p, drive)) != GC_OK) break;
-        if ((rc = launch_wallvel(f, st, p)) != GC_OK) break;
+        if ((rc = launch_walls(f, st, p, f->a.vel)) != GC_OK) break;
     } while (0);
     f->capturing = false;
     cudaGraph_t graph = nullptr;
@@ -2360,6 +2455,13 @@ int finalize_cells(GcFused* f) {
     return GC_OK;
 }
 
+// Lanes per particle of the list passes for n particles.  Measured, us per
+// step with 1 / 2 / 4 / 8 lanes: 6 k channel 174 / 118 / 101 / 97, 16 k fluid
+// 124 / 87 / 76 / 76, 26 k channel 182 / 131 / 118 / 115, 78 k channel
+// 179 / 166 / 165 / 177, 85 k fluid 168 / 161 / 158 / 171, 148 k fluid
+// 225 / 226 / 237 / 263, 524 k suspension 700 / 724 / 773 / 882.
+int pass_lanes(int n) { return n < 40000 ? 8 : (n < 100000 ? 4 : (n < 130000 ? 2 : 1)); }
+
 bool same_physics(const Structconst& a, const Structconst& b) {
     return a.CutRadius == b.CutRadius && a.Mass == b.Mass && a.SoundSpeed1 == b.SoundSpeed1 &&
            a.SoundSpeed2 == b.SoundSpeed2 && a.DenInit == b.DenInit && a.VVsigma == b.VVsigma &&
@@ -2699,7 +2801,12 @@ int gc_ensemble_create(int nsys, const GcSystemDesc* d, int noise_on, const GcFu
         m0 += c.nCellPar;
     }
     f->has_b1 = false;
-    for (const SysInfo& S : f->hsys) f->has_b1 = f->has_b1 || S.b2 > S.id0;
+    for (SysInfo& S : f->hsys) {
+        f->has_b1 = f->has_b1 || S.b2 > S.id0;
+        S.w0 = (unsigned)f->nwall;
+        f->nwall += (int)(S.fl - S.b2);
+    }
+    f->lanes = pass_lanes((int)ntot);
     const int n = f->n;
     int ok = GC_OK;
     SlotArrays* sa[2] = {&f->a, &f->b};

@@ -80,6 +80,7 @@ struct SysInfo {
     uint64_t seed;                   // iSeed of the system (pair noise)
     unsigned id0, b2, fl, cs, end;   // first id; first Bound2, fluid and membrane id; one past the last
     unsigned m0;                     // first membrane index (membrane-ordered arrays)
+    unsigned w0;                     // Bound2 particles of the systems before this one
     int cube0;                       // first global cube of the list grid
     int mcube0;                      // first global cube of the aggregation grid
     float gx;                        // body force in x (ConstExtForce)
@@ -208,6 +209,8 @@ struct GcFused {
     bool ens = false;              // kernels read the system table (several systems)
     bool capturing = false;        // a step is being captured: the noise key comes from the device
     bool has_b1 = true;            // some system has Bound1 wall particles
+    int nwall = 0;                 // Bound2 wall particles of all systems
+    int lanes = 1;                 // lanes per particle of the list passes (pass_lanes)
     long long step = -1;           // index keying the noise of the latest step
     long long rebuilds = 0, steps = 0;
     cudaStream_t st = 0;
@@ -359,6 +362,7 @@ int launch_tile_density(GcFused* f, cudaStream_t st, const GcParams& p, bool mar
 int launch_tile_force(GcFused* f, cudaStream_t st, const GcParams& p, int drive, bool mark);
 int wall_lists(GcFused* f, cudaStream_t st, const float4* bpos, bool host);
 bool any_bound2(const GcFused* f);
+int launch_walls(GcFused* f, cudaStream_t st, const GcParams& p, float4* v);
 void prof_mark(GcFused* f, cudaStream_t st);
 struct SysInfo;
 

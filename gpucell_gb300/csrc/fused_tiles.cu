@@ -538,14 +538,6 @@ __global__ void fk_tile_ffinish(int n, GcParams p, SysInfo s0, const SysInfo* __
     vel[i] = make_float4(h.x + sc * f.x, h.y + sc * f.y, h.z + sc * f.z, 0.f);
 }
 
-// Wall velocity of the Bound2 slots (K10) from their lists of mobile
-// neighbours: v_w = 2 VelHalf - sum v W / sum W, reading and writing `v`.
-template <bool ENS>
-__global__ void fk_tile_wallvel(int n, GcParams p, SysInfo s0, const SysInfo* __restrict__ sys,
-                                const int* __restrict__ sysid, const float4* __restrict__ pos, float4* __restrict__ v,
-                                const float4* __restrict__ vh, const int* __restrict__ nbr,
-                                const int* __restrict__ cnt, int cap);
-
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
@@ -662,12 +654,7 @@ int tile_density_launch(GcFused* f, cudaStream_t st, const GcParams& p) {
     fk_tile_dfinish<ENS><<<gc_blocks(n, f->block), f->block, 0, st>>>(n, p, f->hsys[0], f->dsys, f->a.sys, f->a.pos,
                                                                       f->keys, f->bmask, f->pd, f->dp);
     GC_CHECK_LAUNCH("fused: tile density finish");
-    if (any_bound2(f)) {
-        fk_tile_wallvel<ENS><<<gc_blocks(n, f->block), f->block, 0, st>>>(n, p, f->hsys[0], f->dsys, f->a.sys,
-                                                                          f->a.pos, f->a.vpred, f->a.vh, f->nbr,
-                                                                          f->cnt, f->cap);
-        GC_CHECK_LAUNCH("fused: tile wall velocity");
-    }
+    GC_TRY(launch_walls(f, st, p, f->a.vpred));
     return GC_OK;
 }
 
@@ -699,36 +686,6 @@ int launch_tile_force(GcFused* f, cudaStream_t st, const GcParams& p, int drive,
     GC_TRY(f->ens ? tile_force_launch<true>(f, st, p, drive) : tile_force_launch<false>(f, st, p, drive));
     if (mark) prof_mark(f, st);
     return GC_OK;
-}
-
-template <bool ENS>
-__global__ void fk_tile_wallvel(int n, GcParams p, SysInfo s0, const SysInfo* __restrict__ sys,
-                                const int* __restrict__ sysid, const float4* __restrict__ pos, float4* __restrict__ v,
-                                const float4* __restrict__ vh, const int* __restrict__ nbr,
-                                const int* __restrict__ cnt, int cap) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 xi4 = pos[i];
-    GC_SYS_OF(S, i);
-    if (stype(fid(xi4), S) != PT_B2) return;
-    const Box B = box_of(S);
-    const float3 xi = xyz(xi4);
-    float3 num = f3(0.f, 0.f, 0.f);
-    float den = 0.f;
-    const int c = cnt[i];
-    for (int k = 0; k < c; ++k) {
-        const int j = __ldg(nbr + sell(i, k, cap));
-        const float r2 = norm2_rn(pair_image(xi, xyz(pos[j]), B));
-        if (r2 >= p.rc2) continue;
-        const float w = wendland_w(r2 > 0.f ? r2 * rsqrtf(r2) : 0.f, p);
-        const float4 vj = v[j];
-        num += w * f3(vj.x, vj.y, vj.z);
-        den += w;
-    }
-    const float4 w4 = vh[i];
-    const float3 r = den > 0.f ? f3(2.f * w4.x - num.x / den, 2.f * w4.y - num.y / den, 2.f * w4.z - num.z / den)
-                               : f3(w4.x, w4.y, w4.z);
-    v[i] = make_float4(r.x, r.y, r.z, 0.f);
 }
 
 }  // namespace gcf

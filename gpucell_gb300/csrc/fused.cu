@@ -824,70 +824,117 @@ __device__ __forceinline__ float3 mdiff(const float4* mpos, const float4* mplo, 
 }
 
 
-// Triangle geometry and per-cell area/volume (FP64 sums), one block per cell.
-__global__ void fk_mgeo(GcParams p, const SysInfo* __restrict__ sys, const int* __restrict__ cellsys, int ncell,
-                        int ntri, const int3* __restrict__ tri, const int2* __restrict__ betri,
-                        const float4* __restrict__ mpos, const float4* __restrict__ mplo,
-                        const int4* __restrict__ mnt, float* __restrict__ tarea,
-                        float4* __restrict__ tnorm, float4* __restrict__ tcen, float* __restrict__ reftarea,
-                        double* __restrict__ carea, double* __restrict__ cvol, double* __restrict__ crefarea,
-                        double* __restrict__ crefvol, int setup, unsigned* flags) {
+// The membrane passes go by blocks of kMembBS triangles, several to a cell:
+// one block per cell took 65 us for the geometry and 53 us for the triangle
+// forces of sixteen 5120-triangle cells, on 16 of the 152 SMs and longer than
+// the density pass they run beside.
+constexpr int kMembBS = 128;
+
+// Geometry of the triangles of block blk (block cb.y of cell cb.x) and their
+// share of the cell's area and volume (FP64, relative to the cell's
+// first vertex), to be added in the order of the blocks.
+__device__ __forceinline__ void tri_geometry(int blk, int2 cb, const GcParams& p,
+                                             const SysInfo* __restrict__ sys, const int* __restrict__ cellsys, int ntri,
+                                             const int3* __restrict__ tri, const int2* __restrict__ betri,
+                                             const float4* __restrict__ mpos, const float4* __restrict__ mplo,
+                                             const int4* __restrict__ mnt, float* __restrict__ tarea,
+                                             float4* __restrict__ tnorm, float4* __restrict__ tcen,
+                                             float* __restrict__ reftarea, double2* __restrict__ cpart, int setup,
+                                             unsigned* flags) {
     __shared__ double sh[32];
-    int c = blockIdx.x;
-    int2 be = betri[c];
+    const int c = cb.x, chunk = cb.y;
+    const int2 be = betri[c];
     if (be.x < 0 || be.y >= ntri || be.y < be.x) {
         if (threadIdx.x == 0) raise_flag(flags, GC_FLAG_BAD_INDEX);
         return;
     }
     const GcGrid& g = sys[cellsys ? cellsys[c] : 0].g;
-    int ncp = (int)p.nCP;
-    int r = tri[be.x].x - 1;
+    const int ncp = (int)p.nCP;
+    const int r = tri[be.x].x - 1;
     if (r < 0 || r >= ncp) {
         if (threadIdx.x == 0) raise_flag(flags, GC_FLAG_BAD_INDEX);
         return;
     }
-    float4 xr = mpos[r];
-    int4 tr = mnt[r];
+    const float4 xr = mpos[r];
+    const int4 tr = mnt[r];
     float3 xru = f3(xr.x, xr.y, xr.z);
     if (g.pmask & 1) xru.x += (float)tr.x * g.L[0];
     if (g.pmask & 2) xru.y += (float)tr.y * g.L[1];
     if (g.pmask & 4) xru.z += (float)tr.z * g.L[2];
     double accA = 0.0, accV = 0.0;
-    for (int t = be.x + threadIdx.x; t <= be.y; t += blockDim.x) {
-        int3 v = tri[t];
-        int a = v.x - 1, b = v.y - 1, cc = v.z - 1;
+    const int t = be.x + chunk * kMembBS + (int)threadIdx.x;
+    if (t <= be.y) {
+        const int3 v = tri[t];
+        const int a = v.x - 1, b = v.y - 1, cc = v.z - 1;
         if (a < 0 || b < 0 || cc < 0 || a >= ncp || b >= ncp || cc >= ncp) {
             raise_flag(flags, GC_FLAG_BAD_INDEX);
             tarea[t] = 0.f;
-            continue;
+        } else {
+            const float3 u1 = mdiff(mpos, mplo, mnt, a, r, g);
+            const float3 e1 = mdiff(mpos, mplo, mnt, b, a, g), e2 = mdiff(mpos, mplo, mnt, cc, a, g);
+            const float3 xi = cross3(e1, e2);
+            const float len = sqrtf(dot3(xi, xi));
+            const float A = 0.5f * len;
+            const float3 nrm = len > 0.f ? (1.f / len) * xi : f3(0.f, 0.f, 0.f);
+            const float3 u2 = u1 + e1, u3 = u1 + e2;
+            tarea[t] = A;
+            tnorm[t] = make_float4(nrm.x, nrm.y, nrm.z, 0.f);
+            const float3 cen = xru + (1.f / 3.f) * (u1 + u2 + u3);
+            tcen[t] = make_float4(cen.x, cen.y, cen.z, 0.f);
+            if (setup) reftarea[t] = A;
+            accA = (double)A;
+            const double v1x = u1.x, v1y = u1.y, v1z = u1.z, v2x = u2.x, v2y = u2.y, v2z = u2.z, v3x = u3.x, v3y = u3.y,
+                         v3z = u3.z;
+            accV = (v1x * (v2y * v3z - v2z * v3y) + v1y * (v2z * v3x - v2x * v3z) + v1z * (v2x * v3y - v2y * v3x)) / 6.0;
         }
-        float3 u1 = mdiff(mpos, mplo, mnt, a, r, g);
-        float3 e1 = mdiff(mpos, mplo, mnt, b, a, g), e2 = mdiff(mpos, mplo, mnt, cc, a, g);
-        float3 xi = cross3(e1, e2);
-        float len = sqrtf(dot3(xi, xi));
-        float A = 0.5f * len;
-        float3 nrm = len > 0.f ? (1.f / len) * xi : f3(0.f, 0.f, 0.f);
-        float3 u2 = u1 + e1, u3 = u1 + e2;
-        tarea[t] = A;
-        tnorm[t] = make_float4(nrm.x, nrm.y, nrm.z, 0.f);
-        float3 cen = xru + (1.f / 3.f) * (u1 + u2 + u3);
-        tcen[t] = make_float4(cen.x, cen.y, cen.z, 0.f);
-        if (setup) reftarea[t] = A;
-        accA += (double)A;
-        // volume relative to the cell's first vertex, in FP64
-        double v1x = u1.x, v1y = u1.y, v1z = u1.z, v2x = u2.x, v2y = u2.y, v2z = u2.z, v3x = u3.x, v3y = u3.y,
-               v3z = u3.z;
-        accV += (v1x * (v2y * v3z - v2z * v3y) + v1y * (v2z * v3x - v2x * v3z) + v1z * (v2x * v3y - v2y * v3x)) / 6.0;
     }
-    double Ac = block_sum_d(accA, sh);
-    double Vc = block_sum_d(accV, sh);
+    const double Ac = block_sum_d(accA, sh), Vc = block_sum_d(accV, sh);
+    if (threadIdx.x == 0) cpart[blk] = make_double2(Ac, Vc);
+}
+
+// Area and volume of cell c from the partial sums of its blocks, by the
+// lanes of one warp in a fixed order.
+__device__ __forceinline__ void cell_sums(int c, const int* __restrict__ mfirst, const double2* __restrict__ cpart,
+                                          double* A, double* V) {
+    double a = 0.0, v = 0.0;
+    for (int k = mfirst[c] + (int)(threadIdx.x & 31); k < mfirst[c + 1]; k += 32) {
+        const double2 x = cpart[k];
+        a += x.x;
+        v += x.y;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+    }
+    *A = a;
+    *V = v;
+}
+
+// Set-up geometry: the triangles, then (fk_mref, one warp per cell) the
+// reference area and volume of the cells.
+__global__ void fk_mgeo_setup(GcParams p, const SysInfo* __restrict__ sys, const int* __restrict__ cellsys,
+                              const int2* __restrict__ mblk, int ntri, const int3* __restrict__ tri,
+                              const int2* __restrict__ betri, const float4* __restrict__ mpos, const float4* __restrict__ mplo,
+                              const int4* __restrict__ mnt, float* __restrict__ tarea, float4* __restrict__ tnorm,
+                              float4* __restrict__ tcen, float* __restrict__ reftarea, double2* __restrict__ cpart,
+                              unsigned* flags) {
+    tri_geometry(blockIdx.x, mblk[blockIdx.x], p, sys, cellsys, ntri, tri, betri, mpos, mplo, mnt,
+                 tarea, tnorm, tcen, reftarea, cpart, 1, flags);
+}
+
+__global__ void fk_mref(int ntri, const int2* __restrict__ betri, const int* __restrict__ mfirst,
+                        const double2* __restrict__ cpart,
+                        double* __restrict__ carea, double* __restrict__ cvol, double* __restrict__ crefarea,
+                        double* __restrict__ crefvol) {
+    const int c = blockIdx.x;
+    const int2 be = betri[c];
+    if (be.x < 0 || be.y >= ntri || be.y < be.x) return;
+    double A, V;
+    cell_sums(c, mfirst, cpart, &A, &V);
     if (threadIdx.x == 0) {
-        carea[c] = Ac;
-        cvol[c] = Vc;
-        if (setup) {
-            crefarea[c] = Ac;
-            crefvol[c] = Vc;
-        }
+        carea[c] = crefarea[c] = A;
+        cvol[c] = crefvol[c] = V;
     }
 }
 
@@ -962,12 +1009,11 @@ __global__ void fk_mech_setup(GcParams p, const SysInfo* __restrict__ sys, const
 // -- and with them the whole step -- are the same from run to run.
 __device__ __forceinline__ float4 part(float3 f) { return make_float4(f.x, f.y, f.z, 0.f); }
 
-__global__ void fk_medge(GcParams p, const SysInfo* __restrict__ sys, const int* __restrict__ msys, int nedge,
-                         const int6* __restrict__ edge, const float4* __restrict__ mpos,
+__device__ __forceinline__ void edge_force(int e, const GcParams& p, const SysInfo* __restrict__ sys,
+                         const int* __restrict__ msys, int nedge, const int6* __restrict__ edge, const float4* __restrict__ mpos,
                          const float4* __restrict__ mplo, const int4* __restrict__ mnt, const float* __restrict__ l0a, const float* __restrict__ lmax, const float* __restrict__ perlen,
                          const float* __restrict__ hpow, const float* __restrict__ refang,
                          const float* __restrict__ hbend, float4* __restrict__ parts, unsigned* flags) {
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nedge) return;
     int a, b, c, d;
     float4* out = parts + 4 * (size_t)e;
@@ -1025,43 +1071,91 @@ __global__ void fk_medge(GcParams p, const SysInfo* __restrict__ sys, const int*
     out[3] = part(f4);
 }
 
-__global__ void fk_mtri(GcParams p, const SysInfo* __restrict__ sys, const int* __restrict__ cellsys, int ncell,
-                        const int2* __restrict__ betri, const int3* __restrict__ tri, const float4* __restrict__ mpos,
-                        const float4* __restrict__ mplo, const int4* __restrict__ mnt,
-                        const float* __restrict__ reftarea,
-                        const float* __restrict__ hl, const float* __restrict__ hg, const float* __restrict__ hv,
-                        const double* __restrict__ carea, const double* __restrict__ cvol,
-                        const double* __restrict__ crefarea, const double* __restrict__ crefvol,
-                        float4* __restrict__ parts, int ntri) {
-    // one block per cell: the cell's coefficients are read once
-    int c = blockIdx.x;
-    int2 be = betri[c];
+// Triangle geometry (the first geo_blocks blocks) and edge forces (the
+// others) in one launch: neither needs the other.
+__global__ void __launch_bounds__(kMembBS) fk_mgeo_edge(GcParams p, const SysInfo* __restrict__ sys,
+                                                        const int* __restrict__ cellsys, const int* __restrict__ msys,
+                                                        int geo_blocks, const int2* __restrict__ mblk, int ntri,
+                                                        const int3* __restrict__ tri, const int2* __restrict__ betri,
+                                                        const float4* __restrict__ mpos,
+                                                        const float4* __restrict__ mplo, const int4* __restrict__ mnt,
+                                                        float* __restrict__ tarea, float4* __restrict__ tnorm,
+                                                        float4* __restrict__ tcen, double2* __restrict__ cpart,
+                                                        int nedge, const int6* __restrict__ edge,
+                                                        const float* __restrict__ l0a, const float* __restrict__ lmax,
+                                                        const float* __restrict__ perlen,
+                                                        const float* __restrict__ hpow,
+                                                        const float* __restrict__ refang,
+                                                        const float* __restrict__ hbend, float4* __restrict__ parts,
+                                                        unsigned* flags) {
+    if ((int)blockIdx.x < geo_blocks)
+        tri_geometry(blockIdx.x, mblk[blockIdx.x], p, sys, cellsys, ntri, tri, betri, mpos, mplo,
+                     mnt, tarea, tnorm, tcen, nullptr, cpart, 0, flags);
+    else
+        edge_force((blockIdx.x - geo_blocks) * kMembBS + threadIdx.x, p, sys, msys, nedge, edge, mpos, mplo, mnt, l0a,
+                   lmax, perlen, hpow, refang, hbend, parts, flags);
+}
+
+// Triangle forces; each block adds its cell's area and volume from the
+// partial sums (at most a few dozen), the first one stores them.
+__global__ void __launch_bounds__(kMembBS) fk_mtri(GcParams p, const SysInfo* __restrict__ sys,
+                                                   const int* __restrict__ cellsys, const int2* __restrict__ mblk,
+                                                   const int* __restrict__ mfirst, const int2* __restrict__ betri, const int3* __restrict__ tri,
+                                                   const float4* __restrict__ mpos, const float4* __restrict__ mplo,
+                                                   const int4* __restrict__ mnt, const float* __restrict__ reftarea,
+                                                   const float* __restrict__ hl, const float* __restrict__ hg,
+                                                   const float* __restrict__ hv, const double2* __restrict__ cpart,
+                                                   double* __restrict__ carea, double* __restrict__ cvol,
+                                                   const double* __restrict__ crefarea,
+                                                   const double* __restrict__ crefvol, float4* __restrict__ parts,
+                                                   int ntri) {
+    __shared__ float sd[2];
+    const int2 cb = mblk[blockIdx.x];
+    const int c = cb.x, chunk = cb.y;
+    const int2 be = betri[c];
     if (be.x < 0 || be.y >= ntri || be.y < be.x) return;
-    const GcGrid& g = sys[cellsys ? cellsys[c] : 0].g;
-    float dA = (float)((carea[c] - crefarea[c]) / crefarea[c]);
-    float dV = (float)((cvol[c] - crefvol[c]) / crefvol[c]);
-    int ncp = (int)p.nCP;
-    for (int t = be.x + threadIdx.x; t <= be.y; t += blockDim.x) {
-        int3 v = tri[t];
-        int a = v.x - 1, b = v.y - 1, cc = v.z - 1;
-        float4* out = parts + 3 * (size_t)t;
-        out[0] = out[1] = out[2] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (a < 0 || b < 0 || cc < 0 || a >= ncp || b >= ncp || cc >= ncp) continue;
-        float3 x2 = mdiff(mpos, mplo, mnt, b, a, g), x3 = mdiff(mpos, mplo, mnt, cc, a, g);
-        float3 xi = cross3(x2, x3);
-        float len = sqrtf(dot3(xi, xi));
-        if (!(len > 0.f)) continue;
-        float At = 0.5f * len;
-        float3 nh = (1.f / len) * xi;
-        float A0t = reftarea[t];
-        float cA = hg[t] * dA + hl[t] * (At - A0t) / A0t;
-        float cV = hv[t] * dV * (1.f / 6.f);
-        float3 g1 = 0.5f * cross3(nh, x3 - x2), g2 = 0.5f * cross3(nh, -x3), g3 = 0.5f * cross3(nh, x2);
-        float3 fv = -cV * xi;
-        out[0] = part(fv - cA * g1);
-        out[1] = part(fv - cA * g2);
-        out[2] = part(fv - cA * g3);
+    if (threadIdx.x < 32) {
+        double A, V;
+        cell_sums(c, mfirst, cpart, &A, &V);
+        if (threadIdx.x == 0) {
+            sd[0] = (float)((A - crefarea[c]) / crefarea[c]);
+            sd[1] = (float)((V - crefvol[c]) / crefvol[c]);
+            if (chunk == 0) {
+                carea[c] = A;
+                cvol[c] = V;
+            }
+        }
     }
+    __syncthreads();
+    const float dA = sd[0], dV = sd[1];
+    const GcGrid& g = sys[cellsys ? cellsys[c] : 0].g;
+    const int ncp = (int)p.nCP;
+    const int t = be.x + chunk * kMembBS + (int)threadIdx.x;
+    if (t > be.y) return;
+    const int3 v = tri[t];
+    const int a = v.x - 1, b = v.y - 1, cc = v.z - 1;
+    float4* out = parts + 3 * (size_t)t;
+    float3 f1 = f3(0.f, 0.f, 0.f), f2 = f1, f3v = f1;
+    if (a >= 0 && b >= 0 && cc >= 0 && a < ncp && b < ncp && cc < ncp) {
+        const float3 x2 = mdiff(mpos, mplo, mnt, b, a, g), x3 = mdiff(mpos, mplo, mnt, cc, a, g);
+        const float3 xi = cross3(x2, x3);
+        const float len = sqrtf(dot3(xi, xi));
+        if (len > 0.f) {
+            const float At = 0.5f * len;
+            const float3 nh = (1.f / len) * xi;
+            const float A0t = reftarea[t];
+            const float cA = hg[t] * dA + hl[t] * (At - A0t) / A0t;
+            const float cV = hv[t] * dV * (1.f / 6.f);
+            const float3 g1 = 0.5f * cross3(nh, x3 - x2), g2 = 0.5f * cross3(nh, -x3), g3 = 0.5f * cross3(nh, x2);
+            const float3 fv = -cV * xi;
+            f1 = fv - cA * g1;
+            f2 = fv - cA * g2;
+            f3v = fv - cA * g3;
+        }
+    }
+    out[0] = part(f1);
+    out[1] = part(f2);
+    out[2] = part(f3v);
 }
 
 // Per vertex: the sum of its edge and triangle parts (in the fixed order of
@@ -1074,12 +1168,26 @@ __global__ void fk_mgather(int ncp, int nedge, const int* __restrict__ inc_ptr, 
     if (v >= ncp) return;
     float3 f = f3(0.f, 0.f, 0.f);
     float a = 0.f;
-    const int tri0 = 4 * nedge;
-    for (int q = inc_ptr[v]; q < inc_ptr[v + 1]; ++q) {
-        int k = inc[q];
-        float4 x = parts[k];
-        f += f3(x.x, x.y, x.z);
-        if (k >= tri0) a += tarea[(k - tri0) / 3] * (1.f / 3.f);
+    const int tri0 = 4 * nedge, end = inc_ptr[v + 1];
+    // six parts in flight (a vertex of an icosphere has twelve edge parts and
+    // six triangles), added in order
+    constexpr int U = 6;
+    for (int q = inc_ptr[v]; q < end; q += U) {
+        int k[U];
+        float4 x[U];
+        float ar[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) k[u] = q + u < end ? inc[q + u] : -1;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            x[u] = k[u] >= 0 ? parts[k[u]] : make_float4(0.f, 0.f, 0.f, 0.f);
+            ar[u] = k[u] >= tri0 ? tarea[(k[u] - tri0) / 3] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            f += f3(x[u].x, x[u].y, x[u].z);
+            if (k[u] >= tri0) a += ar[u] * (1.f / 3.f);
+        }
     }
     mforce[v] = make_float4(f.x, f.y, f.z, 0.f);
     parea[v] = a;
@@ -1308,9 +1416,19 @@ __global__ void __launch_bounds__(kAggBS) fk_maggl(int ncp, GcParams p, const Sy
         const float3 xi = xyz(mpos[v]);
         const float ai = parea[v];
         const unsigned b = moff[v], e = moff[v + 1];
-        for (unsigned u = b + k; u < e; u += kAggLanes) {
-            const int j = mlist[u];
-            morse_pair<true>(p, g, xi, ai, mpos[j], parea + j, f);
+        // four partners in flight: a chain of index and position loads set
+        // the time of the vertices with hundreds of partners
+        constexpr int U = 4;
+        for (unsigned u = b + k; u < e; u += U * kAggLanes) {
+            int j[U];
+            float4 y[U];
+#pragma unroll
+            for (int w = 0; w < U; ++w) j[w] = u + w * kAggLanes < e ? mlist[u + w * kAggLanes] : -1;
+#pragma unroll
+            for (int w = 0; w < U; ++w) y[w] = j[w] >= 0 ? mpos[j[w]] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int w = 0; w < U; ++w)
+                if (j[w] >= 0) morse_pair<true>(p, g, xi, ai, y[w], parea + j[w], f);
         }
     }
     // the group's partial forces, added by a fixed tree
@@ -1842,19 +1960,15 @@ int launch_density(GcFused* f, cudaStream_t st, const GcParams& p, bool mark) {
 
 int launch_membranes(GcFused* f, cudaStream_t st, const GcParams& p) {
     if (f->ncell <= 0) return GC_OK;
-    fk_mgeo<<<f->ncell, 256, 0, st>>>(p, f->dsys, f->cellsys, f->ncell, f->ntri, f->tri, f->betri, f->mpos, f->mplo,
-                                      f->mnthro,
-                                     f->tarea, f->tnorm, f->tcen, f->reftarea, f->carea, f->cvol, f->crefarea,
-                                     f->crefvol, 0, f->flags);
-    GC_CHECK_LAUNCH("fused: membrane geometry");
-    fk_medge<<<gc_blocks(f->nedge, f->block), f->block, 0, st>>>(p, f->dsys, f->msys, f->nedge, f->edge, f->mpos,
-                                                                 f->mplo, f->mnthro, f->l0, f->lmax, f->perlen, f->hpow, f->refang,
-                                                                 f->hbend, f->mparts, f->flags);
-    GC_CHECK_LAUNCH("fused: membrane edges");
-    fk_mtri<<<f->ncell, 256, 0, st>>>(p, f->dsys, f->cellsys, f->ncell, f->betri, f->tri, f->mpos, f->mplo,
-                                      f->mnthro,
-                                     f->reftarea, f->hl, f->hg, f->hv, f->carea, f->cvol, f->crefarea, f->crefvol,
-                                     f->mparts + 4 * (size_t)f->nedge, f->ntri);
+    const int geo = f->mblocks;
+    fk_mgeo_edge<<<geo + gc_blocks(f->nedge, kMembBS), kMembBS, 0, st>>>(
+        p, f->dsys, f->cellsys, f->msys, geo, f->mblk, f->ntri, f->tri, f->betri, f->mpos, f->mplo, f->mnthro,
+        f->tarea, f->tnorm, f->tcen, f->cpart, f->nedge, f->edge, f->l0, f->lmax, f->perlen, f->hpow, f->refang,
+        f->hbend, f->mparts, f->flags);
+    GC_CHECK_LAUNCH("fused: membrane geometry and edges");
+    fk_mtri<<<geo, kMembBS, 0, st>>>(p, f->dsys, f->cellsys, f->mblk, f->mfirst, f->betri, f->tri, f->mpos, f->mplo,
+                                     f->mnthro, f->reftarea, f->hl, f->hg, f->hv, f->cpart, f->carea, f->cvol, f->crefarea,
+                                     f->crefvol, f->mparts + 4 * (size_t)f->nedge, f->ntri);
     GC_CHECK_LAUNCH("fused: membrane triangles");
     fk_mgather<<<gc_blocks(f->ncp, f->block), f->block, 0, st>>>(f->ncp, f->nedge, f->inc_ptr, f->inc, f->mparts,
                                                                  f->tarea, f->mforce, f->parea);
@@ -2355,6 +2469,27 @@ int build_incidence(GcFused* f, const int* tri, const int* edge) {
     return GC_OK;
 }
 
+// The blocks of the triangle passes from the cells' triangle ranges (host
+// array); a cell with a bad range has one, which reports it.
+int membrane_blocks(GcFused* f, const int* betri) {
+    std::vector<int2> blk;
+    std::vector<int> first((size_t)f->ncell + 1, 0);
+    for (int c = 0; c < f->ncell; ++c) {
+        const int b = betri[2 * (size_t)c], e = betri[2 * (size_t)c + 1];
+        const int nb = b >= 0 && e < f->ntri && e >= b ? (e - b) / kMembBS + 1 : 1;
+        for (int k = 0; k < nb; ++k) blk.push_back(make_int2(c, k));
+        first[(size_t)c + 1] = (int)blk.size();
+    }
+    f->mblocks = (int)blk.size();
+    GC_TRY(falloc(f, &f->mblk, blk.size()));
+    GC_TRY(falloc(f, &f->mfirst, first.size()));
+    GC_TRY(falloc(f, &f->cpart, blk.size()));
+    GC_CUDA(cudaMemcpyAsync(f->mblk, blk.data(), blk.size() * sizeof(int2), cudaMemcpyHostToDevice, f->st), "fused: cells");
+    GC_CUDA(cudaMemcpyAsync(f->mfirst, first.data(), first.size() * 4, cudaMemcpyHostToDevice, f->st), "fused: cells");
+    GC_CUDA(cudaStreamSynchronize(f->st), "fused: cells");   // the host vectors go out of scope
+    return GC_OK;
+}
+
 // Concatenates the systems' topologies with global vertex, triangle and cell
 // offsets and uploads them.
 int finalize_cells(GcFused* f) {
@@ -2417,6 +2552,7 @@ int finalize_cells(GcFused* f) {
     GC_TRY(up(f->hl, hl.data(), hl.size() * 4));
     GC_TRY(up(f->hg, hg.data(), hg.size() * 4));
     GC_TRY(up(f->hv, hv.data(), hv.size() * 4));
+    GC_TRY(membrane_blocks(f, betri.data()));
     GC_TRY(build_incidence(f, tri.data(), edge.data()));
     {
         std::vector<int> cv(2 * (size_t)ncell);
@@ -3013,10 +3149,13 @@ int gc_fused_setup(GcFused* f) {
         fk_gather_mpos<<<gc_blocks(f->ncp, 256), 256, 0, st>>>(f->ncp, f->dsys, f->msys, f->slot_of, f->a.pos,
                                                               f->a.nthro, f->a.plo, f->mpos, f->mplo, f->mnthro);
         GC_CHECK_LAUNCH("fused: membrane positions");
-        fk_mgeo<<<f->ncell, 256, 0, st>>>(p, f->dsys, f->cellsys, f->ncell, f->ntri, f->tri, f->betri, f->mpos,
-                                         f->mplo, f->mnthro, f->tarea, f->tnorm, f->tcen, f->reftarea, f->carea, f->cvol,
-                                         f->crefarea, f->crefvol, 1, f->flags);
+        fk_mgeo_setup<<<f->mblocks, kMembBS, 0, st>>>(
+            p, f->dsys, f->cellsys, f->mblk, f->ntri, f->tri, f->betri, f->mpos, f->mplo, f->mnthro, f->tarea,
+            f->tnorm, f->tcen, f->reftarea, f->cpart, f->flags);
         GC_CHECK_LAUNCH("fused: set-up geometry");
+        fk_mref<<<f->ncell, 32, 0, st>>>(f->ntri, f->betri, f->mfirst, f->cpart, f->carea, f->cvol, f->crefarea,
+                                         f->crefvol);
+        GC_CHECK_LAUNCH("fused: reference areas and volumes");
         fk_mech_setup<<<gc_blocks(f->nedge, f->block), f->block, 0, st>>>(
             p, f->dsys, f->msys, f->nedge, f->edge, f->mpos, f->mplo, f->mnthro, f->shear, f->bend, f->l0, f->lmax, f->perlen,
             f->hpow, f->hbend, f->refang, f->flags);

@@ -160,7 +160,10 @@ int engine_cells(GcFused* f, const GcRefPtrs& r) {
     std::vector<int> htri(3 * (size_t)ntri), hedge(6 * (size_t)nedge);
     GC_CUDA(cudaMemcpyAsync(htri.data(), f->tri, htri.size() * 4, cudaMemcpyDeviceToHost, st), "fused engine: topology");
     GC_CUDA(cudaMemcpyAsync(hedge.data(), f->edge, hedge.size() * 4, cudaMemcpyDeviceToHost, st), "fused engine: topology");
+    std::vector<int> hbetri(2 * (size_t)ncell);
+    GC_CUDA(cudaMemcpyAsync(hbetri.data(), f->betri, hbetri.size() * 4, cudaMemcpyDeviceToHost, st), "fused engine: topology");
     GC_CUDA(cudaStreamSynchronize(st), "fused engine: topology");
+    GC_TRY(membrane_blocks(f, hbetri.data()));
     GC_TRY(build_incidence(f, htri.data(), hedge.data()));
     return build_grids(f);   // aggregation grid
 }

@@ -306,6 +306,10 @@ struct GcFused {
     float *l0 = nullptr, *lmax = nullptr, *perlen = nullptr, *hpow = nullptr, *hbend = nullptr, *refang = nullptr;
     float *tarea = nullptr, *reftarea = nullptr;
     float4 *tnorm = nullptr, *tcen = nullptr;
+    int mblocks = 0;             // blocks of kMembBS triangles of all cells
+    int2* mblk = nullptr;        // of each: its cell and its place among the cell's blocks
+    int* mfirst = nullptr;       // first block of each cell (ncell + 1)
+    double2* cpart = nullptr;    // area and volume partial sums of each block
     double *carea = nullptr, *cvol = nullptr, *crefarea = nullptr, *crefvol = nullptr;
     float4 *mpos = nullptr, *mforce = nullptr, *magg = nullptr;
     float4* mplo = nullptr;      // low parts of mpos (the double-float positions of the membrane vertices)
@@ -384,6 +388,7 @@ int restore_state(GcFused* f, StateCopy* c);
 int refresh(GcFused* f);
 int alloc_cells(GcFused* f, int ncell, int ntri, int nedge, int ncp);
 int build_incidence(GcFused* f, const int* tri, const int* edge);
+int membrane_blocks(GcFused* f, const int* betri);
 int check_sys(GcFused* f, int sys, const char* what);
 int store_range(GcFused* f, unsigned id_base, int count, float* pos, float* vel, float* rho, float* press,
                 float* force, float* velhalf, int* nthro, int to_device);

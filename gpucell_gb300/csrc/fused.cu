@@ -410,7 +410,8 @@ __device__ __forceinline__ void wall_velocity(int q, int nwall, int n, const GcP
                                               const SysInfo* __restrict__ sys, int nsys,
                                               const int* __restrict__ slot_of, const float4* __restrict__ pos,
                                               float4* __restrict__ v, const float4* __restrict__ vh,
-                                              const int* __restrict__ nbr, const int* __restrict__ cnt, int cap) {
+                                              const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
+                                              PairRec* __restrict__ rec) {
     const int w = q / kWallLanes, s = q % kWallLanes;
     if (w >= nwall) return;   // whole groups
     int k0 = 0;
@@ -455,6 +456,7 @@ __device__ __forceinline__ void wall_velocity(int q, int nwall, int n, const GcP
     const float3 r = den > 0.f ? f3(2.f * w4.x - num.x / den, 2.f * w4.y - num.y / den, 2.f * w4.z - num.z / den)
                                : f3(w4.x, w4.y, w4.z);
     v[i] = make_float4(r.x, r.y, r.z, 0.f);
+    if (rec) rec[i] = PairRec{pos[i], make_float4(r.x, r.y, r.z, p.mass / p.rho0)};
 }
 
 template <bool ENS>
@@ -463,7 +465,7 @@ __global__ void fk_wallvel(int nwall, int n, GcParams p, SysInfo s0, const SysIn
                            const float4* __restrict__ vh, const int* __restrict__ nbr, const int* __restrict__ cnt,
                            int cap) {
     wall_velocity<ENS>(blockIdx.x * blockDim.x + threadIdx.x, nwall, n, p, s0, sys, nsys, slot_of, pos, v, vh, nbr, cnt,
-                       cap);
+                       cap, nullptr);
 }
 
 #ifndef GC_DENS_MIN_BLOCKS
@@ -480,10 +482,11 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
                                                   float2* __restrict__ dp, const int* __restrict__ nbr,
                                                   const int* __restrict__ cnt, int cap, unsigned* __restrict__ cmask,
                                                   int mw, int* __restrict__ ccnt, float wrap_margin, int wall_blocks,
-                                                  int nwall, int nsys, const int* __restrict__ slot_of) {
+                                                  int nwall, int nsys, const int* __restrict__ slot_of,
+                                                  PairRec* __restrict__ rec) {
     if ((int)blockIdx.x < wall_blocks) {
         wall_velocity<ENS>(blockIdx.x * blockDim.x + threadIdx.x, nwall, n, p, s0, sys, nsys, slot_of, pos, vpred, vh,
-                           nbr, cnt, cap);
+                           nbr, cnt, cap, rec);
         return;
     }
     const int q = (blockIdx.x - wall_blocks) * blockDim.x + threadIdx.x;
@@ -497,7 +500,10 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
     const unsigned b2 = S.b2;
     int t = stype(id, S);
     if (t != PT_FLUID && t != PT_MEMB) {
-        if (s == 0) dp[i] = make_float2(p.mass / p.rho0, 0.f);
+        if (s == 0) {
+            dp[i] = make_float2(p.mass / p.rho0, 0.f);
+            if (t == PT_B1) rec[i] = PairRec{xi4, make_float4(0.f, 0.f, 0.f, p.mass / p.rho0)};
+        }
         return;
     }
     const unsigned gm = group_mask<L>();
@@ -551,7 +557,7 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
                     acc += in && sdpd ? t2 * t2 * fmaf(r, inv_rc4, 1.f) : 0.f;
                     // acting: an SDPD partner within rc, or a Bound1 wall within the repulsion range
                     const bool act = in && apart && (sdpd || (B1 && r2 < p.rep_r0sq));
-                    m |= (unsigned)act << (k0 - w0 + u);
+                    m |= act ? 0x80000000u >> (k0 - w0 + u) : 0u;
                 }
             }
             if (cmask) {
@@ -574,6 +580,8 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
     float c2 = (t == PT_MEMB) ? p.c2sq : p.c1sq;
     float inv_d = __frcp_rn(sum);
     dp[i] = make_float2(inv_d, c2 * (rho - p.rho0) * inv_d * inv_d);
+    const float4 vp = vpred[i];
+    rec[i] = PairRec{xi4, make_float4(vp.x, vp.y, vp.z, inv_d)};
 }
 
 // ---------------------------------------------------------------------------
@@ -587,19 +595,9 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
 // next group are loaded while the current group is evaluated, and a group's
 // position, density and velocity loads are issued together, so that each
 // thread has several independent gathers in flight.
-#ifndef GC_FORCE_GROUP
-#define GC_FORCE_GROUP 1
-#endif
-#ifndef GC_FORCE_AHEAD
-#define GC_FORCE_AHEAD 1
-#endif
-constexpr int kForceGroup = GC_FORCE_GROUP;
-constexpr int kForceAhead = GC_FORCE_AHEAD;   // groups of list indices loaded ahead
-
-#ifndef GC_FORCE_MIN_BLOCKS
-#define GC_FORCE_MIN_BLOCKS (kForceGroup == 1 ? 6 : (kForceGroup == 2 ? 4 : 3))
-#endif
-constexpr int force_min_blocks(bool ens) { return GC_FORCE_MIN_BLOCKS - (ens ? 1 : 0); }
+constexpr int kForceGroup = 1;
+constexpr int kForceAhead = 1;   // groups of list indices loaded ahead
+constexpr int force_min_blocks(bool ens) { return ens ? 5 : 6; }
 
 // The predicted velocity of a neighbour packed to FP16 (x, y | z, 0): 8 bytes
 // per gather instead of 16 (GcFusedOptions.half_velocity, an experiment).
@@ -617,21 +615,37 @@ __global__ void fk_pack_vel(int n, const float4* __restrict__ v, uint2* __restri
     out[i] = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
 }
 
+// The ten round keys of the step's pair noise.  A host-driven step of one
+// system passes them in the kernel's parameters, where each round takes its
+// key from the constant bank; ensembles and captured steps, whose key is on
+// the device, add them up pair by pair (ten instructions).
+struct PhiloxKeys {
+    uint32_t k[10];
+};
+
+__device__ __forceinline__ PairRec load_rec(const PairRec* p) {
+    PairRec r;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.x.x), "=f"(r.x.y), "=f"(r.x.z), "=f"(r.x.w), "=f"(r.v.x), "=f"(r.v.y), "=f"(r.v.z), "=f"(r.v.w)
+        : "l"(p));
+    return r;
+}
+
 // L lanes per particle take even shares of its entries (ranks c s / L to
 // c (s + 1) / L), in the order of the list.
-template <bool COMPACT, bool ENS, bool HALFV, bool NOISE, bool B1, int L>
+template <bool COMPACT, bool ENS, bool HALFV, bool NOISE, bool B1, int L, bool KEYS>
 __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
     fk_force(int n, GcParams p, SysInfo s0, const SysInfo* __restrict__ sys, const int* __restrict__ sysid,
-             const unsigned* __restrict__ nkey, const float4* __restrict__ pos, const float4* __restrict__ vpred,
-             const float4* __restrict__ vh, const float2* __restrict__ dp, float4* __restrict__ force,
-             float4* __restrict__ vel, const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
+             const unsigned* __restrict__ nkey, const PairRec* __restrict__ rec, const float4* __restrict__ vh,
+             const float2* __restrict__ dp, float4* __restrict__ force, float4* __restrict__ vel, const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
              const unsigned* __restrict__ cmask, int mw, const float4* __restrict__ mforce, int drive,
-             const uint2* __restrict__ vph, float wrap_margin) {
+             const uint2* __restrict__ vph, float wrap_margin, PhiloxKeys pk) {
     constexpr int G = L > 1 ? 2 : kForceGroup;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = q / L, ln = q % L;
     if (i >= n) return;
-    float4 xi4 = pos[i];
+    const PairRec ri = load_rec(rec + i);
+    const float4 xi4 = ri.x;
     float3 xi = xyz(xi4);
     unsigned id = fid(xi4);
     const int s = ENS ? (sysid ? sysid[i] : 0) : 0;
@@ -642,13 +656,14 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
     }
     const Box B = box_of(S);
     const unsigned b2 = S.b2;
-    const unsigned id0 = S.id0;
-    // one system: the key of the step from the parameters, or, in a captured
-    // step, from the device (fk_step_begin derives it at each replay)
-    const uint32_t key = ENS ? nkey[s] : (nkey ? nkey[0] : p.noise_key);
-    float4 vi = vpred[i];
-    float2 dpi = dp[i];
-    float3 f = f3(0.f, 0.f, 0.f);
+    const unsigned id0 = ENS ? S.id0 : 0u;
+    // without KEYS the key of the step comes from the device (fk_step_begin
+    // derives it, in a captured step at each replay)
+    const uint32_t key = !NOISE || KEYS ? 0u : nkey[s];
+    const float4 vi = ri.v;
+    const float pti = dp[i].y;
+    float2 fxy = make_float2(0.f, 0.f);
+    float fz = 0.f;
     const int call = cnt[i];
     const int first = call * ln / L;                     // this lane's entries
     const int c = call * (ln + 1) / L - first;
@@ -667,7 +682,7 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
             r -= here;
         }
         if (c > 0)
-            for (; r > 0; --r) m &= m - 1;
+            for (; r > 0; --r) m &= ~(0x80000000u >> __clz(m));
     }
     // index of the next acting entry (COMPACT) or of the next entry; called
     // once per entry, in order.  The scan for a non-empty mask word ends: it
@@ -686,8 +701,8 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
                 base += 32;
                 m = __ldg(mp + (size_t)(base >> 5) * 32);
             }
-            int b = __ffs(m) - 1;
-            m &= m - 1;
+            const int b = __clz(m);
+            m &= ~(0x80000000u >> b);
             return base + b;
         } else {
             return first + k;
@@ -700,40 +715,70 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
     // along v_ij (viscous) and one along xi_ij (random).  F (d_i^-1 d_j^-1)
     // is formed as F times the product of the two inverse number densities,
     // the same product from either side of the pair.
+    // x and y go through packed instructions (one for both), z beside them:
+    // with the round keys from the constant bank 244 M warp instructions at 524 k
+    // particles against 253 M unpacked.
     const float cAB = p.sqrtAB - p.sqrtA;
-    // one pair: neighbour position (with its id), (1/d, P/d^2) and velocity
-    auto pair = [&](auto wrapc, float4 xj4, float2 dpj, float4 vj) {
+    auto add_f = [&](float c, float2 axy, float az) {   // f += c a
+        fxy = __ffma2_rn(make_float2(c, c), axy, fxy);
+        fz = fmaf(c, az, fz);
+    };
+    // one pair: the neighbour's record and P/d^2
+    auto pair = [&](auto wrapc, PairRec rj, float ptj) {
         constexpr bool W = decltype(wrapc)::value;
-        float3 d = pair_diff<W>(xi, xyz(xj4), B);
-        float r2 = norm2_fma(d);   // as in fk_density
+        float2 dxy;
+        float dz;
+        if constexpr (W) {
+            const float3 d = pair_image(xi, xyz(rj.x), B);
+            dxy = make_float2(d.x, d.y);
+            dz = d.z;
+        } else {
+            dxy = __ffma2_rn(make_float2(rj.x.x, rj.x.y), make_float2(-1.f, -1.f), make_float2(xi.x, xi.y));
+            dz = __fsub_rn(xi.z, rj.x.z);
+        }
+        const float r2 = fmaf(dxy.x, dxy.x, fmaf(dxy.y, dxy.y, dz * dz));   // as in fk_density
         if (!COMPACT && (r2 >= p.rc2 || r2 <= 0.f)) return;   // coincident pairs exert no force
-        unsigned idj = fid(xj4);
-        float inv_r = rsqrt_ftz(r2);
+        const unsigned idj = fid(rj.x);
+        const float inv_r = rsqrt_ftz(r2), ir2 = inv_r * inv_r;
         if (B1 && idj < b2) {   // Bound1: repulsion only (B1: some system has such walls)
             if (r2 < p.rep_r0sq) {
-                float ir2 = inv_r * inv_r;
-                float q2 = p.rep_r0sq * ir2, q4 = q2 * q2, q12 = q4 * q4 * q4;
-                f += (p.rep_D * (q12 - q4) * ir2) * d;
+                const float q2 = p.rep_r0sq * ir2, q4 = q2 * q2, q12 = q4 * q4 * q4;
+                add_f(p.rep_D * (q12 - q4) * ir2, dxy, dz);
             }
             return;
         }
-        float F = wendland_f(r2 * inv_r, p);
-        float ir2 = inv_r * inv_r;
-        float3 vij = f3(vi.x - vj.x, vi.y - vj.y, vi.z - vj.z);
-        float fdd = F * (dpi.x * dpj.x);
-        float cd = (dpi.y + dpj.y) * F - (fdd * p.visB) * dot3(d, vij) * ir2;
-        f += (-fdd * p.visA) * vij;
+        const float F = wendland_f(r2 * inv_r, p);
+        const float2 vxy = __ffma2_rn(make_float2(rj.v.x, rj.v.y), make_float2(-1.f, -1.f), make_float2(vi.x, vi.y));
+        const float vz = vi.z - rj.v.z;
+        const float fdd = F * (vi.w * rj.v.w);
+        const float dv = fmaf(dxy.x, vxy.x, fmaf(dxy.y, vxy.y, dz * vz));
+        float cd = (pti + ptj) * F - (fdd * p.visB) * dv * ir2;
+        add_f(-fdd * p.visA, vxy, vz);
         if constexpr (NOISE) {
-            float qq = p.noise_pref * fdd;
-            float q = qq > 0.f ? qq * rsqrt_ftz(qq) : 0.f;
+            // (a pair at the cut-off can give F a rounding-sized negative value: no noise then)
+            const float qq = fmaxf(p.noise_pref * fdd, 1e-36f);
+            float q = qq * rsqrt_ftz(qq);
             q = id < idj ? q : -q;   // the pair sign of xi_ij
-            float3 xi_ = pair_noise_unsigned_k(id - id0, idj - id0, key);
-            cd += (q * cAB) * dot3(d, xi_) * ir2;
-            f += (q * p.sqrtA) * xi_;
+            const unsigned ia = id - id0, ib = idj - id0;
+            const Philox2 w = philox2x32_10_keys(min(ia, ib), max(ia, ib), [&](int r) {
+                return KEYS ? pk.k[r] : key + 0x9E3779B9u * (unsigned)r;
+            });
+            const float3 xi_ = unit_uniforms(w);
+            const float dx = fmaf(dxy.x, xi_.x, fmaf(dxy.y, xi_.y, dz * xi_.z));
+            cd += (q * cAB) * dx * ir2;
+            add_f(q * p.sqrtA, make_float2(xi_.x, xi_.y), xi_.z);
         }
-        f += cd * d;
+        add_f(cd, dxy, dz);
     };
-    auto gather_v = [&](int j) -> float4 { return HALFV ? unpack_vel(vph[j]) : vpred[j]; };
+    auto gather = [&](int j) -> PairRec {
+        PairRec r = load_rec(rec + j);
+        if constexpr (HALFV) {
+            const float w = r.v.w;
+            r.v = unpack_vel(vph[j]);
+            r.v.w = w;
+        }
+        return r;
+    };
     auto run = [&](auto wrapc) {
         {
             int jq[A][G];
@@ -745,13 +790,12 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
                     jq[a][u] = k < c ? __ldg(lp + (size_t)next_k(k) * 32) : i;
                 }
             for (int k0 = 0; k0 < c; k0 += G) {
-                float4 xg[G], vg[G];
-                float2 dg[G];
+                PairRec rg[G];
+                float pg[G];
 #pragma unroll
                 for (int u = 0; u < G; ++u) {
-                    xg[u] = pos[jq[0][u]];
-                    dg[u] = dp[jq[0][u]];
-                    vg[u] = gather_v(jq[0][u]);
+                    rg[u] = gather(jq[0][u]);
+                    pg[u] = dp[jq[0][u]].y;
                 }
 #pragma unroll
                 for (int a = 0; a + 1 < A; ++a)
@@ -765,7 +809,7 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
 #pragma unroll
                 for (int u = 0; u < G; ++u) {
                     if (k0 + u >= c) break;
-                    pair(wrapc, xg[u], dg[u], vg[u]);
+                    pair(wrapc, rg[u], pg[u]);
                 }
             }
         }
@@ -775,6 +819,7 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
     // every listed pair there); any other warp forms the image.
     if (__any_sync(__activemask(), near_face(xi, S.g, wrap_margin))) run(std::true_type{});
     else run(std::false_type{});
+    float3 f = f3(fxy.x, fxy.y, fz);
     if constexpr (L > 1) {
         const unsigned gm = group_mask<L>();
         f = f3(group_sum<L>(f.x, gm), group_sum<L>(f.y, gm), group_sum<L>(f.z, gm));
@@ -1935,7 +1980,7 @@ void density_launch(GcFused* f, cudaStream_t st, const GcParams& p, unsigned* cm
     auto go = [&](auto ens, auto b1) {
         fk_density<decltype(ens)::value, decltype(b1)::value, L><<<nb, bs, 0, st>>>(
             f->n, p, s0(f), f->dsys, f->a.sys, f->a.pos, f->a.vpred, f->a.vh, f->dp, f->nbr, f->cnt, f->cap, cm, f->mw,
-            cc, wrap_margin(f), wb, f->nwall, f->nsys, f->slot_of);
+            cc, wrap_margin(f), wb, f->nwall, f->nsys, f->slot_of, f->rec);
     };
     if (f->ens) {
         if (f->has_b1) go(std::true_type{}, std::true_type{});
@@ -1990,14 +2035,16 @@ void force_launch_n(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
     const int* c = COMPACT ? f->ccnt : f->cnt;
     const unsigned* cm = COMPACT ? f->cmask : nullptr;
     const unsigned* nk = f->ens || f->capturing ? f->nkey : nullptr;
-    if (f->ens)
-        fk_force<COMPACT, true, HALFV, NOISE, B1, L><<<nb, f->block, 0, st>>>(
-            n, p, s0(f), f->dsys, f->a.sys, nk, f->a.pos, f->a.vpred, f->a.vh, f->dp, f->a.force, f->a.vel,
-            f->nbr, c, f->cap, cm, f->mw, mf, drive, f->vph, wrap_margin(f));
-    else
-        fk_force<COMPACT, false, HALFV, NOISE, B1, L><<<nb, f->block, 0, st>>>(
-            n, p, s0(f), f->dsys, f->a.sys, nk, f->a.pos, f->a.vpred, f->a.vh, f->dp, f->a.force, f->a.vel,
-            f->nbr, c, f->cap, cm, f->mw, mf, drive, f->vph, wrap_margin(f));
+    PhiloxKeys pk;
+    for (int r = 0; r < 10; ++r) pk.k[r] = p.noise_key + 0x9E3779B9u * (unsigned)r;
+    auto go = [&](auto ens, auto keys) {
+        fk_force<COMPACT, decltype(ens)::value, HALFV, NOISE, B1, L, decltype(keys)::value><<<nb, f->block, 0, st>>>(
+            n, p, s0(f), f->dsys, f->a.sys, nk, f->rec, f->a.vh, f->dp, f->a.force, f->a.vel, f->nbr, c, f->cap, cm,
+            f->mw, mf, drive, f->vph, wrap_margin(f), pk);
+    };
+    if (f->ens) go(std::true_type{}, std::false_type{});
+    else if (NOISE && !nk) go(std::false_type{}, std::bool_constant<NOISE>{});
+    else go(std::false_type{}, std::false_type{});
 }
 
 template <bool COMPACT, bool HALFV, int L>
@@ -2958,6 +3005,7 @@ int gc_ensemble_create(int nsys, const GcSystemDesc* d, int noise_on, const GcFu
     }
     if (ok == GC_OK) ok = falloc(f, &f->refpos, n);
     if (ok == GC_OK) ok = falloc(f, &f->dp, n);
+    if (ok == GC_OK) ok = falloc(f, &f->rec, n);
     if (ok == GC_OK) ok = falloc(f, &f->vph, (size_t)n + 1);
     if (ok == GC_OK) ok = falloc(f, &f->slot_of, n);
     if (ok == GC_OK) ok = falloc(f, &f->keys, n > f->ncp ? n : f->ncp);

@@ -155,6 +155,14 @@ struct SlotArrays {
     int* sys;   // system of each slot (nullptr for one system)
 };
 
+// What the force pass gathers of a neighbour, written by the density pass:
+// position and id, predicted velocity and 1/d in one 32-byte record, which
+// one 256-bit load brings in.  P/d^2 comes from the (1/d, P/d^2) array.
+struct __align__(32) PairRec {
+    float4 x;   // position, id bits
+    float4 v;   // predicted velocity, 1/d
+};
+
 // Membrane topology of one system as given (local, 1-based), until set-up.
 struct HostCells {
     bool set = false;
@@ -218,6 +226,7 @@ struct GcFused {
     gcf::SlotArrays a{}, b{};
     float4* refpos = nullptr;
     float2* dp = nullptr;
+    gcf::PairRec* rec = nullptr;   // per slot, for the force pass of the same step
     int* slot_of = nullptr;
     int *keys = nullptr, *vals = nullptr;
     int *nbr = nullptr, *cnt = nullptr;

@@ -206,7 +206,9 @@ struct Philox2 {
     uint32_t w0, w1;
 };
 
-__host__ __device__ __forceinline__ Philox2 philox2x32_10(uint32_t c0, uint32_t c1, uint32_t k) {
+// key(r) is the key of round r: k + r 0x9E3779B9.
+template <class Key>
+__host__ __device__ __forceinline__ Philox2 philox2x32_10_keys(uint32_t c0, uint32_t c1, Key&& key) {
 #ifdef __CUDA_ARCH__
 #pragma unroll
 #endif
@@ -214,11 +216,14 @@ __host__ __device__ __forceinline__ Philox2 philox2x32_10(uint32_t c0, uint32_t 
         // one 32x32 -> 64-bit product gives both halves
         uint64_t pr = (uint64_t)0xD256D193u * c0;
         uint32_t hi = (uint32_t)(pr >> 32), lo = (uint32_t)pr;
-        c0 = hi ^ k ^ c1;
+        c0 = hi ^ key(r) ^ c1;
         c1 = lo;
-        k += 0x9E3779B9u;
     }
     return Philox2{c0, c1};
+}
+
+__host__ __device__ __forceinline__ Philox2 philox2x32_10(uint32_t c0, uint32_t c1, uint32_t k) {
+    return philox2x32_10_keys(c0, c1, [k](int r) { return k + 0x9E3779B9u * (uint32_t)r; });
 }
 
 // Three uniform variates with zero mean and unit variance from the 63 low
@@ -228,9 +233,14 @@ __host__ __device__ __forceinline__ Philox2 philox2x32_10(uint32_t c0, uint32_t 
 // device the 21 bits become the mantissa of a float in [1, 2), v = 1 + u/2^21,
 // and the variate is sqrt(12) v - sqrt(12) (3/2 - 2^-22): no int-to-float
 // conversion.
-__device__ __forceinline__ float unit_uniform21(uint32_t u) {
-    float v = __uint_as_float(0x3F800000u | (u << 2));
+// `b` holds the 21 bits from bit 2 on (its other bits are ignored).
+__device__ __forceinline__ float unit_uniform21(uint32_t b) {
+    const float v = __uint_as_float((b & 0x7FFFFCu) | 0x3F800000u);
     return fmaf(v, 3.4641016151377544f, -3.4641016151377544f * (1.5f - 2.384185791015625e-7f));
+}
+
+__device__ __forceinline__ float3 unit_uniforms(Philox2 w) {
+    return f3(unit_uniform21(w.w0 << 2), unit_uniform21(__funnelshift_r(w.w0, w.w1, 19)), unit_uniform21(w.w1 >> 8));
 }
 
 // The noise components xi_ij for the pair (i, j) without the sign of the
@@ -238,11 +248,7 @@ __device__ __forceinline__ float unit_uniform21(uint32_t u) {
 __device__ __forceinline__ float3 pair_noise_unsigned_k(unsigned id_i, unsigned id_j, uint32_t key) {
     unsigned a = id_i < id_j ? id_i : id_j;
     unsigned b = id_i < id_j ? id_j : id_i;
-    Philox2 w = philox2x32_10(a, b, key);
-    uint32_t u0 = w.w0 & 0x1FFFFFu;
-    uint32_t u1 = (w.w0 >> 21) | ((w.w1 & 0x3FFu) << 11);
-    uint32_t u2 = (w.w1 >> 10) & 0x1FFFFFu;
-    return f3(unit_uniform21(u0), unit_uniform21(u1), unit_uniform21(u2));
+    return unit_uniforms(philox2x32_10(a, b, key));
 }
 
 __device__ __forceinline__ float3 pair_noise_unsigned(unsigned id_i, unsigned id_j, const GcParams& p) {

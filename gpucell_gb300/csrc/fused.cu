@@ -637,7 +637,7 @@ template <bool COMPACT, bool ENS, bool HALFV, bool NOISE, bool B1, int L, bool K
 __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
     fk_force(int n, GcParams p, SysInfo s0, const SysInfo* __restrict__ sys, const int* __restrict__ sysid,
              const unsigned* __restrict__ nkey, const PairRec* __restrict__ rec, const float4* __restrict__ vh,
-             const float2* __restrict__ dp, float4* __restrict__ force, float4* __restrict__ vel, const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
+             float4* __restrict__ force, float4* __restrict__ vel, const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
              const unsigned* __restrict__ cmask, int mw, const float4* __restrict__ mforce, int drive,
              const uint2* __restrict__ vph, float wrap_margin, PhiloxKeys pk) {
     constexpr int G = L > 1 ? 2 : kForceGroup;
@@ -661,7 +661,16 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
     // derives it, in a captured step at each replay)
     const uint32_t key = !NOISE || KEYS ? 0u : nkey[s];
     const float4 vi = ri.v;
-    const float pti = dp[i].y;
+    // P/d^2 of a particle from w = 1/d and its squared sound speed:
+    // c^2 (rho - rho0) / d^2 = c^2 w (m - rho0 w), zero at rho0 (walls) to a
+    // rounding.  Three operations instead of a second gather per pair, which
+    // took a fifth of the pass's L1 wavefronts.  Where all sound speeds are
+    // one, B1 is false or c1sq = c2sq.
+    auto pterm = [&](float w, unsigned pid) -> float {
+        const float c2 = B1 ? (pid >= S.cs ? p.c2sq : p.c1sq) : p.c1sq;
+        return (c2 * w) * fmaf(-p.rho0, w, p.mass);
+    };
+    const float pti = pterm(ri.v.w, id);
     float2 fxy = make_float2(0.f, 0.f);
     float fz = 0.f;
     const int call = cnt[i];
@@ -715,16 +724,17 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
     // along v_ij (viscous) and one along xi_ij (random).  F (d_i^-1 d_j^-1)
     // is formed as F times the product of the two inverse number densities,
     // the same product from either side of the pair.
-    // x and y go through packed instructions (one for both), z beside them:
-    // with the round keys from the constant bank 244 M warp instructions at 524 k
-    // particles against 253 M unpacked.
+    // The velocity difference goes through a packed instruction (x and y in
+    // one), as the record's load leaves them in a register pair; packing the
+    // sums as well cost more moves than it saved (266 M against 253 M warp
+    // instructions at 524 k particles).
     const float cAB = p.sqrtAB - p.sqrtA;
     auto add_f = [&](float c, float2 axy, float az) {   // f += c a
-        fxy = __ffma2_rn(make_float2(c, c), axy, fxy);
+        fxy = make_float2(fmaf(c, axy.x, fxy.x), fmaf(c, axy.y, fxy.y));
         fz = fmaf(c, az, fz);
     };
-    // one pair: the neighbour's record and P/d^2
-    auto pair = [&](auto wrapc, PairRec rj, float ptj) {
+    // one pair: the neighbour's record
+    auto pair = [&](auto wrapc, PairRec rj) {
         constexpr bool W = decltype(wrapc)::value;
         float2 dxy;
         float dz;
@@ -733,7 +743,7 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
             dxy = make_float2(d.x, d.y);
             dz = d.z;
         } else {
-            dxy = __ffma2_rn(make_float2(rj.x.x, rj.x.y), make_float2(-1.f, -1.f), make_float2(xi.x, xi.y));
+            dxy = make_float2(xi.x - rj.x.x, xi.y - rj.x.y);
             dz = __fsub_rn(xi.z, rj.x.z);
         }
         const float r2 = fmaf(dxy.x, dxy.x, fmaf(dxy.y, dxy.y, dz * dz));   // as in fk_density
@@ -752,12 +762,11 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
         const float vz = vi.z - rj.v.z;
         const float fdd = F * (vi.w * rj.v.w);
         const float dv = fmaf(dxy.x, vxy.x, fmaf(dxy.y, vxy.y, dz * vz));
-        float cd = (pti + ptj) * F - (fdd * p.visB) * dv * ir2;
+        float cd = (pti + pterm(rj.v.w, idj)) * F - (fdd * p.visB) * dv * ir2;
         add_f(-fdd * p.visA, vxy, vz);
         if constexpr (NOISE) {
-            // (a pair at the cut-off can give F a rounding-sized negative value: no noise then)
-            const float qq = fmaxf(p.noise_pref * fdd, 1e-36f);
-            float q = qq * rsqrt_ftz(qq);
+            // (a pair at the cut-off can give F a rounding-sized negative value: its noise is as small)
+            float q = sqrt_ftz(fabsf(p.noise_pref * fdd));
             q = id < idj ? q : -q;   // the pair sign of xi_ij
             const unsigned ia = id - id0, ib = idj - id0;
             const Philox2 w = philox2x32_10_keys(min(ia, ib), max(ia, ib), [&](int r) {
@@ -791,12 +800,8 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
                 }
             for (int k0 = 0; k0 < c; k0 += G) {
                 PairRec rg[G];
-                float pg[G];
 #pragma unroll
-                for (int u = 0; u < G; ++u) {
-                    rg[u] = gather(jq[0][u]);
-                    pg[u] = dp[jq[0][u]].y;
-                }
+                for (int u = 0; u < G; ++u) rg[u] = gather(jq[0][u]);
 #pragma unroll
                 for (int a = 0; a + 1 < A; ++a)
 #pragma unroll
@@ -809,7 +814,7 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
 #pragma unroll
                 for (int u = 0; u < G; ++u) {
                     if (k0 + u >= c) break;
-                    pair(wrapc, rg[u], pg[u]);
+                    pair(wrapc, rg[u]);
                 }
             }
         }
@@ -2039,7 +2044,7 @@ void force_launch_n(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
     for (int r = 0; r < 10; ++r) pk.k[r] = p.noise_key + 0x9E3779B9u * (unsigned)r;
     auto go = [&](auto ens, auto keys) {
         fk_force<COMPACT, decltype(ens)::value, HALFV, NOISE, B1, L, decltype(keys)::value><<<nb, f->block, 0, st>>>(
-            n, p, s0(f), f->dsys, f->a.sys, nk, f->rec, f->a.vh, f->dp, f->a.force, f->a.vel, f->nbr, c, f->cap, cm,
+            n, p, s0(f), f->dsys, f->a.sys, nk, f->rec, f->a.vh, f->a.force, f->a.vel, f->nbr, c, f->cap, cm,
             f->mw, mf, drive, f->vph, wrap_margin(f), pk);
     };
     if (f->ens) go(std::true_type{}, std::false_type{});
@@ -2050,7 +2055,7 @@ void force_launch_n(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
 template <bool COMPACT, bool HALFV, int L>
 void force_launch_l(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
     const bool noise = p.noise_pref > 0.f;
-    if (f->has_b1) {
+    if (f->has_b1 || p.c1sq != p.c2sq) {   // B1: some system has Bound1 walls, or two sound speeds
         if (noise) force_launch_n<COMPACT, HALFV, true, true, L>(f, st, p, drive);
         else force_launch_n<COMPACT, HALFV, false, true, L>(f, st, p, drive);
     } else {

@@ -157,7 +157,7 @@ struct SlotArrays {
 
 // What the force pass gathers of a neighbour, written by the density pass:
 // position and id, predicted velocity and 1/d in one 32-byte record, which
-// one 256-bit load brings in.  P/d^2 comes from the (1/d, P/d^2) array.
+// one 256-bit load brings in.
 struct __align__(32) PairRec {
     float4 x;   // position, id bits
     float4 v;   // predicted velocity, 1/d

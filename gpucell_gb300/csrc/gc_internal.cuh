@@ -127,6 +127,13 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     return y;
 }
 
+// sqrt(x) by the hardware approximation (PTX sqrt.approx.ftz.f32).
+__device__ __forceinline__ float sqrt_ftz(float x) {
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // |d|^2 with fused multiply-adds: the form the fused step's pair passes use
 // (one rounding fewer than norm2_rn; both passes of a step form it alike).
 __device__ __forceinline__ float norm2_fma(float3 d) { return fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z)); }

@@ -463,7 +463,8 @@ template <bool ENS>
 __global__ void fk_wallvel(int nwall, int n, GcParams p, SysInfo s0, const SysInfo* __restrict__ sys, int nsys,
                            const int* __restrict__ slot_of, const float4* __restrict__ pos, float4* __restrict__ v,
                            const float4* __restrict__ vh, const int* __restrict__ nbr, const int* __restrict__ cnt,
-                           int cap) {
+                           int cap, const int* __restrict__ skip) {
+    if (skip && *skip) return;
     wall_velocity<ENS>(blockIdx.x * blockDim.x + threadIdx.x, nwall, n, p, s0, sys, nsys, slot_of, pos, v, vh, nbr, cnt,
                        cap, nullptr);
 }
@@ -472,6 +473,9 @@ __global__ void fk_wallvel(int nwall, int n, GcParams p, SysInfo s0, const SysIn
 #define GC_DENS_MIN_BLOCKS 5
 #endif
 
+// A pass with `skip` set does nothing where that word is non-zero: it was
+// queued before the host knew that the lists have to be rebuilt first.
+//
 // The first `wall_blocks` blocks give the Bound2 particles their velocity
 // (first, as theirs are the longest chains), the others take L lanes per
 // particle.
@@ -483,7 +487,8 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
                                                   const int* __restrict__ cnt, int cap, unsigned* __restrict__ cmask,
                                                   int mw, int* __restrict__ ccnt, float wrap_margin, int wall_blocks,
                                                   int nwall, int nsys, const int* __restrict__ slot_of,
-                                                  PairRec* __restrict__ rec) {
+                                                  PairRec* __restrict__ rec, const int* __restrict__ skip) {
+    if (skip && *skip) return;
     if ((int)blockIdx.x < wall_blocks) {
         wall_velocity<ENS>(blockIdx.x * blockDim.x + threadIdx.x, nwall, n, p, s0, sys, nsys, slot_of, pos, vpred, vh,
                            nbr, cnt, cap, rec);
@@ -639,7 +644,9 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
              const unsigned* __restrict__ nkey, const PairRec* __restrict__ rec, const float4* __restrict__ vh,
              float4* __restrict__ force, float4* __restrict__ vel, const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
              const unsigned* __restrict__ cmask, int mw, const float4* __restrict__ mforce, int drive,
-             const uint2* __restrict__ vph, float wrap_margin, PhiloxKeys pk) {
+             const uint2* __restrict__ vph, float wrap_margin, PhiloxKeys pk,
+             const int* __restrict__ skip) {
+    if (skip && *skip) return;
     constexpr int G = L > 1 ? 2 : kForceGroup;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = q / L, ln = q % L;
@@ -1985,7 +1992,7 @@ void density_launch(GcFused* f, cudaStream_t st, const GcParams& p, unsigned* cm
     auto go = [&](auto ens, auto b1) {
         fk_density<decltype(ens)::value, decltype(b1)::value, L><<<nb, bs, 0, st>>>(
             f->n, p, s0(f), f->dsys, f->a.sys, f->a.pos, f->a.vpred, f->a.vh, f->dp, f->nbr, f->cnt, f->cap, cm, f->mw,
-            cc, wrap_margin(f), wb, f->nwall, f->nsys, f->slot_of, f->rec);
+            cc, wrap_margin(f), wb, f->nwall, f->nsys, f->slot_of, f->rec, f->skip);
     };
     if (f->ens) {
         if (f->has_b1) go(std::true_type{}, std::true_type{});
@@ -2045,7 +2052,7 @@ void force_launch_n(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
     auto go = [&](auto ens, auto keys) {
         fk_force<COMPACT, decltype(ens)::value, HALFV, NOISE, B1, L, decltype(keys)::value><<<nb, f->block, 0, st>>>(
             n, p, s0(f), f->dsys, f->a.sys, nk, f->rec, f->a.vh, f->a.force, f->a.vel, f->nbr, c, f->cap, cm,
-            f->mw, mf, drive, f->vph, wrap_margin(f), pk);
+            f->mw, mf, drive, f->vph, wrap_margin(f), pk, f->skip);
     };
     if (f->ens) go(std::true_type{}, std::false_type{});
     else if (NOISE && !nk) go(std::false_type{}, std::bool_constant<NOISE>{});
@@ -2104,10 +2111,10 @@ int launch_walls(GcFused* f, cudaStream_t st, const GcParams& p, float4* v) {
     const int nb = gc_blocks((long long)f->nwall * kWallLanes, f->block);
     if (f->ens)
         fk_wallvel<true><<<nb, f->block, 0, st>>>(f->nwall, f->n, p, s0(f), f->dsys, f->nsys, f->slot_of, f->a.pos, v,
-                                                  f->a.vh, f->nbr, f->cnt, f->cap);
+                                                  f->a.vh, f->nbr, f->cnt, f->cap, f->skip);
     else
         fk_wallvel<false><<<nb, f->block, 0, st>>>(f->nwall, f->n, p, s0(f), f->dsys, f->nsys, f->slot_of, f->a.pos, v,
-                                                   f->a.vh, f->nbr, f->cnt, f->cap);
+                                                   f->a.vh, f->nbr, f->cnt, f->cap, f->skip);
     GC_CHECK_LAUNCH("fused: wall velocity");
     return GC_OK;
 }
@@ -2137,7 +2144,37 @@ int join_membranes(GcFused* f, cudaStream_t st) {
 
 int early_store(GcFused* f, cudaStream_t st, int phase);
 
-// One step on the host-driven path: the host reads the rebuild flag.
+// The passes of a step after the integration and any rebuild; `hooks`: with
+// the output hooks and the profiling marks.
+int passes(GcFused* f, const GcParams& p, int drive, bool hooks) {
+    cudaStream_t st = f->st;
+    // the membrane passes beside the density pass (after a rebuild, which
+    // writes the Morse lists they read)
+    GC_TRY(fork_membranes(f, st, f->mst, p));
+    if (hooks && f->early) GC_TRY(f->early(f, st, 0));
+    if (hooks) prof_mark(f, st);
+    GC_TRY(launch_density(f, st, p, true));
+    if (hooks && f->early) GC_TRY(f->early(f, st, 1));
+    if (hooks) prof_mark(f, st);
+    GC_TRY(join_membranes(f, st));
+    if (hooks && f->early) GC_TRY(f->early(f, st, 2));
+    if (hooks) prof_mark(f, st);
+    GC_TRY(launch_force(f, st, p, drive));
+    if (hooks) prof_mark(f, st);
+    GC_TRY(launch_walls(f, st, p, f->a.vel));
+    if (hooks && f->early) GC_TRY(f->early(f, st, 3));
+    return GC_OK;
+}
+
+// One step on the host-driven path: the host reads the rebuild flag.  The
+// passes are queued behind the integration before it has: where the flag
+// turns out set (about one step in ten) the list passes find it set on the
+// device too and do nothing, and the host rebuilds the lists and queues the
+// step's passes again (the membrane passes run twice, with the same results).
+// The GPU then does not wait for the host in every step (15 us of a 90 us
+// step of a 6 thousand particle channel).  Steps with outputs written while
+// they run, with profiling marks and with the pair tiles wait for the flag
+// first.
 int one_step(GcFused* f, int drive) {
     cudaStream_t st = f->st;
     f->step += 1;
@@ -2146,24 +2183,25 @@ int one_step(GcFused* f, int drive) {
     if (f->ens) GC_TRY(launch_step_begin(f, st));
     else GC_CUDA(cudaMemsetAsync(f->rebuild, 0, sizeof(int), st), "fused: flag");
     GC_TRY(launch_integrate(f, st, p));
-    GC_CUDA(cudaMemcpyAsync(&f->h->rebuild, f->rebuild, sizeof(int), cudaMemcpyDeviceToHost, st), "fused: flag");
-    GC_CUDA(cudaStreamSynchronize(st), "fused: flag");
+    const bool ahead = f->lists && !f->early && !f->profile;
+    cudaStream_t fs = ahead ? f->fst : st;
+    if (ahead) {
+        GC_CUDA(cudaEventRecord(f->ev_flag[0], st), "fused: flag");
+        GC_CUDA(cudaStreamWaitEvent(fs, f->ev_flag[0], 0), "fused: flag");
+    }
+    GC_CUDA(cudaMemcpyAsync(&f->h->rebuild, f->rebuild, sizeof(int), cudaMemcpyDeviceToHost, fs), "fused: flag");
+    if (ahead) {
+        GC_CUDA(cudaEventRecord(f->ev_flag[1], fs), "fused: flag");
+        f->skip = f->rebuild;
+        const int rc = passes(f, p, drive, false);
+        f->skip = nullptr;
+        GC_TRY(rc);
+        GC_CUDA(cudaEventSynchronize(f->ev_flag[1]), "fused: flag");
+    } else {
+        GC_CUDA(cudaStreamSynchronize(st), "fused: flag");
+    }
     if (f->h->rebuild) GC_TRY(rebuild_lists(f));
-    // the membrane passes beside the density pass (after a rebuild, which
-    // writes the Morse lists they read)
-    GC_TRY(fork_membranes(f, st, f->mst, p));
-    if (f->early) GC_TRY(f->early(f, st, 0));
-    prof_mark(f, st);
-    GC_TRY(launch_density(f, st, p, true));
-    if (f->early) GC_TRY(f->early(f, st, 1));
-    prof_mark(f, st);
-    GC_TRY(join_membranes(f, st));
-    if (f->early) GC_TRY(f->early(f, st, 2));
-    prof_mark(f, st);
-    GC_TRY(launch_force(f, st, p, drive));
-    prof_mark(f, st);
-    GC_TRY(launch_walls(f, st, p, f->a.vel));
-    if (f->early) GC_TRY(f->early(f, st, 3));
+    if (!ahead || f->h->rebuild) GC_TRY(passes(f, p, drive, true));
     f->steps++;
     return GC_OK;
 }
@@ -3034,7 +3072,10 @@ int gc_ensemble_create(int nsys, const GcSystemDesc* d, int noise_on, const GcFu
         ok = gc_fail(GC_ENOMEM, "fused: pinned words");
     if (ok == GC_OK && (cudaStreamCreateWithFlags(&f->mst, cudaStreamNonBlocking) != cudaSuccess ||
                         cudaEventCreateWithFlags(&f->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-                        cudaEventCreateWithFlags(&f->ev_join, cudaEventDisableTiming) != cudaSuccess))
+                        cudaEventCreateWithFlags(&f->ev_join, cudaEventDisableTiming) != cudaSuccess ||
+                        cudaStreamCreateWithFlags(&f->fst, cudaStreamNonBlocking) != cudaSuccess ||
+                        cudaEventCreateWithFlags(&f->ev_flag[0], cudaEventDisableTiming) != cudaSuccess ||
+                        cudaEventCreateWithFlags(&f->ev_flag[1], cudaEventDisableTiming) != cudaSuccess))
         ok = gc_fail(GC_ECUDA, "fused: membrane stream");
     for (int c = 0; c < 4 && ok == GC_OK; ++c)
         if (cudaEventCreateWithFlags(&f->xev[c], cudaEventDisableTiming) != cudaSuccess)
@@ -3423,6 +3464,10 @@ int gc_fused_destroy(GcFused* f) {
     if (f->gst2) cudaStreamDestroy(f->gst2);
     if (f->gst3) cudaStreamDestroy(f->gst3);
     if (f->mst) cudaStreamDestroy(f->mst);
+    if (f->fst) cudaStreamSynchronize(f->fst);
+    if (f->fst) cudaStreamDestroy(f->fst);
+    for (cudaEvent_t e : f->ev_flag)
+        if (e) cudaEventDestroy(e);
     if (f->ev_fork) cudaEventDestroy(f->ev_fork);
     if (f->ev_join) cudaEventDestroy(f->ev_join);
     for (int c = 0; c < 4; ++c)

@@ -295,6 +295,10 @@ struct GcFused {
     // force pass, beside the rebuild check, the list rebuild and the density.
     cudaStream_t mst = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // the rebuild flag of a host-driven step comes to the host on a stream of
+    // its own, while the passes of the step are queued behind the integration
+    cudaStream_t fst = nullptr;
+    cudaEvent_t ev_flag[2] = {nullptr, nullptr};
     cudaEvent_t xev[4] = {nullptr, nullptr, nullptr, nullptr};   // chunks of a host load / store
     // outputs written while a step runs (gc_fused_step_store, the engine's
     // write-back): called at four points of a host-driven step (0 after the
@@ -336,6 +340,7 @@ struct GcFused {
     bool cells_adopted = false;   // membranes taken from the boundary entry points' buffers
     bool have_agg = false;
     bool setup_done = false;
+    const int* skip = nullptr;    // word that makes the list passes being queued do nothing (one_step)
     // captured steps
     cudaStream_t gst = nullptr, gst2 = nullptr, gst3 = nullptr;
     cudaGraph_t cg[2] = {};

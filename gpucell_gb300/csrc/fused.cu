@@ -241,9 +241,14 @@ __global__ void fk_copy_slots(int n, SlotArrays src, SlotArrays dst) {
     if (dst.sys) dst.sys[q] = src.sys[q];
 }
 
+constexpr int kBuildMinBlocks = 4;   // 64 registers: the build ran 0.554 ms against 0.578 ms unbounded (524k particles)
+
 // Candidates [b, e) of one row of cubes against xs, the image of slot i's
-// position that the row needs; appends the ones within the cut-off to the
-// list of slot i (entry k at lst[32 k]).
+// position that the row needs; with WRITE appends the ones within the cut-off
+// to the list of slot i (entry k at lst[32 k]), otherwise only counts them.
+// ANY: the row may hold slot i itself or candidates that slot i does not list
+// (Bound2 slots list moving particles only), or the list may be full.
+template <bool WRITE, bool ANY>
 __device__ __forceinline__ void scan_range(const float4* __restrict__ pos, unsigned b, unsigned e, float3 xs, int i,
                                            float cut2, bool mobile_only, unsigned fl, int cap,
                                            int* __restrict__ lst, int& k) {
@@ -255,8 +260,9 @@ __device__ __forceinline__ void scan_range(const float4* __restrict__ pos, unsig
         float4 xj = pos[j];
         float dx = xs.x - xj.x, dy = xs.y - xj.y, dz = xs.z - xj.z;
         float r2 = dx * dx + dy * dy + dz * dz;
-        const bool take = r2 < cut2 && (int)j != i && !(mobile_only && fid(xj) < fl);
-        if (take && k < cap) lst[(size_t)k * 32] = (int)j;
+        bool take = r2 < cut2;
+        if (ANY) take = take && (int)j != i && !(mobile_only && fid(xj) < fl);
+        if (WRITE && take && (!ANY || k < cap)) lst[(size_t)k * 32] = (int)j;
         k += take;
     }
 }
@@ -273,89 +279,124 @@ __device__ __forceinline__ float slab_gap(float x, int c, int axis, const GcGrid
     return gap;
 }
 
-// One thread per slot scans the cells of its system's list grid within the
-// stencil radius R around its own (R = 2 for cells at least (rc + skin)/2
-// wide, R = 1 for cubes at least rc + skin wide; either way every pair
-// within rc + skin is found).  Fluid and membrane slots list every particle
-// within rc + skin; Bound2 slots list the moving particles (for their wall
-// velocity); Bound1 slots list nothing.  Positions are inside the box on
-// periodic axes (the permutation wraps them), so each neighbouring row of
-// cells has one image shift, and the 2R + 1 cells of a row that do not wrap
-// are one contiguous range of slots.
-__global__ void __launch_bounds__(kMaxBS, GC_BUILD_MIN_BLOCKS) fk_build_list(int n, const SysInfo* __restrict__ sys,
+// Scans the rows [r0, r1) of the (2R+1)^2 rows of cells around slot i, in its
+// system's list grid (R = 2 for cells at least (rc + skin)/2 wide, R = 1 for
+// cubes at least rc + skin wide; either way every pair within rc + skin is
+// found).  Fluid and membrane slots list every particle within rc + skin;
+// Bound2 slots list the moving particles (for their wall velocity); Bound1
+// slots list nothing.  Positions are inside the box on periodic axes (the
+// permutation wraps them), so each neighbouring row of cells has one image
+// shift, and the 2R + 1 cells of a row that do not wrap are one contiguous
+// range of slots.  Returns k plus the number of entries found.
+//
+// Rows and cells that lie wholly beyond the cut-off are not scanned: the
+// distance from the (image of the) position to a row's y/z slab leaves a
+// reach along x, and only the cells within it are read.  The slabs are taken
+// with a margin far above the rounding of the cell assignment, and the edge
+// cells of a wall axis reach to infinity (particles beyond the grid are
+// clamped into them), so no candidate within the cut-off is skipped and the
+// lists are the same entries in the same order as a scan of all (2R+1)^3 cells.
+//
+// The lanes of a warp wait for one another at the end of each row, which
+// keeps their loads on the same lines: each going through its own rows
+// without waiting, the scan is bound by L1 wavefronts (0.69 against 0.55 ms
+// at 524 k particles).
+template <bool WRITE>
+__device__ __forceinline__ int scan_rows(int r0, int r1, int k, int i, float3 xi, int t, const SysInfo& S,
+                                         const float4* __restrict__ pos, const unsigned* __restrict__ start,
+                                         int* __restrict__ lst, int cap, float cut2) {
+    const GcGrid& g = S.g;
+    const unsigned fl = S.fl;
+    const bool mobile_only = t == PT_B2;
+    const int R = S.lr, side = 2 * R + 1;
+    const int cx = cube_coord(xi.x, 0, g), cy = cube_coord(xi.y, 1, g), cz = cube_coord(xi.z, 2, g);
+    const float cut = sqrtf(cut2), eps = 2e-3f;
+    const float lim2 = (cut + eps) * (cut + eps);
+    for (int r = r0; r < r1; ++r) {
+        const int dz = r / side - R, dy = r % side - R;
+        int z = cz + dz;
+        float sz = 0.f;
+        if (z < 0) { if (!(g.pmask & 4)) continue; z += g.n[2]; sz = g.L[2]; }
+        else if (z >= g.n[2]) { if (!(g.pmask & 4)) continue; z -= g.n[2]; sz = -g.L[2]; }
+        const float dzv = slab_gap(xi.z + sz, z, 2, g);
+        if (dzv * dzv > lim2) continue;
+        int y = cy + dy;
+        float sy = 0.f;
+        if (y < 0) { if (!(g.pmask & 2)) continue; y += g.n[1]; sy = g.L[1]; }
+        else if (y >= g.n[1]) { if (!(g.pmask & 2)) continue; y -= g.n[1]; sy = -g.L[1]; }
+        const float dyv = slab_gap(xi.y + sy, y, 1, g);
+        const float d2 = dyv * dyv + dzv * dzv;
+        if (d2 > lim2) continue;
+        // cells along x within the reach left by this row
+        const float reach = sqrtf(fmaxf(cut2 - d2, 0.f)) + eps;
+        const int xlo = max(cx - R, (int)floorf((xi.x - reach - g.origin[0]) * g.invw[0]));
+        const int xhi = min(cx + R, (int)floorf((xi.x + reach - g.origin[0]) * g.invw[0]));
+        const int row = S.cube0 + g.n[0] * (y + g.n[1] * z);
+        // one range, or near a face of the x axis cell by cell (the edge cells
+        // of a wall axis hold clamped particles: always scanned)
+        const bool whole = xlo >= 0 && xhi < g.n[0];
+        const int a = whole || (g.pmask & 1) ? xlo : cx - R, b = whole || (g.pmask & 1) ? xhi : cx + R;
+        for (int x0 = a; x0 <= b; x0 = whole ? b + 1 : x0 + 1) {
+            int x = x0;
+            float sx = 0.f;
+            if (x < 0) { if (!(g.pmask & 1)) continue; x += g.n[0]; sx = g.L[0]; }
+            else if (x >= g.n[0]) { if (!(g.pmask & 1)) continue; x -= g.n[0]; sx = -g.L[0]; }
+            const unsigned jb = start[row + x], je = start[row + (whole ? b : x) + 1];
+            const float3 xs = f3(xi.x + sx, xi.y + sy, xi.z + sz);
+            if (mobile_only || (dy == 0 && dz == 0) || k + (int)(je - jb) > cap)
+                scan_range<WRITE, true>(pos, jb, je, xs, i, cut2, mobile_only, fl, cap, lst, k);
+            else
+                scan_range<WRITE, false>(pos, jb, je, xs, i, cut2, false, 0u, cap, lst, k);
+        }
+    }
+    return k;
+}
+
+// The lists, by L threads per slot: one thread scans all rows; several take
+// even shares of the rows, count, and scan again to write each its part of
+// the list behind the parts before it (small systems, where a thread's serial
+// scan of 420 candidates sets the time: 102 us for 6 thousand particles, 56
+// with eight threads; from 80 thousand on two scans take longer than one).
+// The lists are the same entries in the same order either way.
+template <int L>
+__global__ void __launch_bounds__(kMaxBS, kBuildMinBlocks) fk_build_list(int n, const SysInfo* __restrict__ sys,
                                                      const int* __restrict__ sysid, const float4* __restrict__ pos,
                                                      const unsigned* __restrict__ start, int* __restrict__ nbr,
                                                      int* __restrict__ cnt, int cap, float cut2, unsigned* flags,
                                                      int* __restrict__ need, int walls_only) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = q / L, ln = q % L;
     if (i >= n) return;
     float4 xi4 = pos[i];
-    float3 xi = xyz(xi4);
     unsigned id = fid(xi4);
     const SysInfo& S = sys[sysid ? sysid[i] : 0];
     int t = stype(id, S);
     if (walls_only && t != PT_B2) {   // the pair tiles cover the other slots
-        cnt[i] = 0;
+        if (ln == 0) cnt[i] = 0;
         return;
     }
-    int k = 0;
-    const GcGrid& g = S.g;
-    const unsigned fl = S.fl;
     int* lst = nbr + sell(i, 0, cap);
-    const bool mobile_only = t == PT_B2;
+    const int rows = (2 * S.lr + 1) * (2 * S.lr + 1);
+    int k = 0;
     if (t != PT_B1) {
-        const int R = S.lr;
-        int cx = cube_coord(xi.x, 0, g), cy = cube_coord(xi.y, 1, g), cz = cube_coord(xi.z, 2, g);
-        // Rows and cells that lie wholly beyond the cut-off are not scanned:
-        // the distance from the (image of the) position to a row's y/z slab
-        // leaves a reach along x, and only the cells within it are read.
-        // The slabs are taken with a margin far above the rounding of the
-        // cell assignment, and the edge cells of a wall axis reach to
-        // infinity (particles beyond the grid are clamped into them), so no
-        // candidate within the cut-off is skipped and the lists are the same
-        // entries in the same order as a scan of all (2R+1)^3 cells.
-        const float cut = sqrtf(cut2), eps = 2e-3f;
-        const float lim2 = (cut + eps) * (cut + eps);
-        for (int dz = -R; dz <= R; ++dz) {
-            int z = cz + dz;
-            float sz = 0.f;
-            if (z < 0) { if (!(g.pmask & 4)) continue; z += g.n[2]; sz = g.L[2]; }
-            else if (z >= g.n[2]) { if (!(g.pmask & 4)) continue; z -= g.n[2]; sz = -g.L[2]; }
-            const float dzv = slab_gap(xi.z + sz, z, 2, g);
-            if (dzv * dzv > lim2) continue;
-            for (int dy = -R; dy <= R; ++dy) {
-                int y = cy + dy;
-                float sy = 0.f;
-                if (y < 0) { if (!(g.pmask & 2)) continue; y += g.n[1]; sy = g.L[1]; }
-                else if (y >= g.n[1]) { if (!(g.pmask & 2)) continue; y -= g.n[1]; sy = -g.L[1]; }
-                const float dyv = slab_gap(xi.y + sy, y, 1, g);
-                const float d2 = dyv * dyv + dzv * dzv;
-                if (d2 > lim2) continue;
-                // cells along x within the reach left by this row
-                const float reach = sqrtf(fmaxf(cut2 - d2, 0.f)) + eps;
-                const int xlo = max(cx - R, (int)floorf((xi.x - reach - g.origin[0]) * g.invw[0]));
-                const int xhi = min(cx + R, (int)floorf((xi.x + reach - g.origin[0]) * g.invw[0]));
-                int row = S.cube0 + g.n[0] * (y + g.n[1] * z);
-                if (xlo >= 0 && xhi < g.n[0]) {
-                    if (xlo <= xhi)
-                        scan_range(pos, start[row + xlo], start[row + xhi + 1], f3(xi.x, xi.y + sy, xi.z + sz), i,
-                                   cut2, mobile_only, fl, cap, lst, k);
-                } else {
-                    // near a face of the x axis: cell by cell (the edge cells
-                    // of a wall axis hold clamped particles: always scanned)
-                    const int a = (g.pmask & 1) ? xlo : cx - R, b = (g.pmask & 1) ? xhi : cx + R;
-                    for (int x0 = a; x0 <= b; ++x0) {
-                        int x = x0;
-                        float sx = 0.f;
-                        if (x < 0) { if (!(g.pmask & 1)) continue; x += g.n[0]; sx = g.L[0]; }
-                        else if (x >= g.n[0]) { if (!(g.pmask & 1)) continue; x -= g.n[0]; sx = -g.L[0]; }
-                        scan_range(pos, start[row + x], start[row + x + 1], f3(xi.x + sx, xi.y + sy, xi.z + sz), i,
-                                   cut2, mobile_only, fl, cap, lst, k);
-                    }
-                }
+        const float3 xi = xyz(xi4);
+        if constexpr (L == 1) {
+            k = scan_rows<true>(0, rows, 0, i, xi, t, S, pos, start, lst, cap, cut2);
+        } else {
+            const int r0 = rows * ln / L, r1 = rows * (ln + 1) / L;
+            const unsigned gm = ((1u << L) - 1u) << ((threadIdx.x & 31) & ~(L - 1));
+            const int c = scan_rows<false>(r0, r1, 0, i, xi, t, S, pos, start, lst, cap, cut2);
+            int end = c;   // inclusive scan over the lanes
+#pragma unroll
+            for (int o = 1; o < L; o <<= 1) {
+                const int v = __shfl_up_sync(gm, end, o, L);
+                if (ln >= o) end += v;
             }
+            k = __shfl_sync(gm, end, L - 1, L);
+            if (c) scan_rows<true>(r0, r1, end - c, i, xi, t, S, pos, start, lst, cap, cut2);
         }
     }
+    if (ln != 0) return;
     if (k > cap) {   // the list holds cap entries; the host grows it to the longest wanted
         raise_flag(flags, GC_FLAG_CELL_OVERFLOW);
         atomicMax(need, k);
@@ -364,7 +405,23 @@ __global__ void __launch_bounds__(kMaxBS, GC_BUILD_MIN_BLOCKS) fk_build_list(int
     cnt[i] = k;
     // pad to a multiple of four with the sentinel slot n (its position is
     // NaN, so it never passes a cut-off test); the capacity is a multiple of 8
-    for (int q = k; q < ((k + 3) & ~3); ++q) nbr[sell(i, q, cap)] = n;
+    for (int e = k; e < ((k + 3) & ~3); ++e) nbr[sell(i, e, cap)] = n;
+}
+
+// The neighbour lists from the positions bpos of the slots and the cube
+// starts of the latest sort; walls_only: of the Bound2 slots, beside the pair
+// tiles.
+int launch_build(GcFused* f, cudaStream_t st, const float4* bpos, int walls_only) {
+    const float cut = f->p.rc + f->skin;
+    const int L = f->lanes == 8 ? 8 : 1, nb = gc_blocks((long long)f->n * L, f->block);
+    auto go = [&](auto kern) {
+        kern<<<nb, f->block, 0, st>>>(f->n, f->dsys, f->a.sys, bpos, f->sb.cnt, f->nbr, f->cnt, f->cap, cut * cut,
+                                      f->oflag, f->need, walls_only);
+    };
+    if (L == 8) go(fk_build_list<8>);
+    else go(fk_build_list<1>);
+    GC_CHECK_LAUNCH("fused: build lists");
+    return GC_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -1929,14 +1986,10 @@ int rebuild_lists(GcFused* f) {
         f->rebuilds++;
         return GC_OK;
     }
-    float cut = f->p.rc + f->skin;
-    float cut2 = cut * cut;
     for (int attempt = 0; attempt < 4; ++attempt) {
         GC_CUDA(cudaMemsetAsync(f->oflag, 0, sizeof(unsigned), st), "fused: flags");
         GC_CUDA(cudaMemsetAsync(f->need, 0, sizeof(int), st), "fused: flags");
-        fk_build_list<<<nb, f->block, 0, st>>>(n, f->dsys, f->a.sys, f->a.pos, f->sb.cnt, f->nbr, f->cnt, f->cap,
-                                              cut2, f->oflag, f->need, 0);
-        GC_CHECK_LAUNCH("fused: build lists");
+        GC_TRY(launch_build(f, st, f->a.pos, 0));
         GC_CUDA(cudaMemcpyAsync(&f->h->oflag, f->oflag, sizeof(unsigned), cudaMemcpyDeviceToHost, st), "fused: flags");
         GC_CUDA(cudaMemcpyAsync(&f->h->need, f->need, sizeof(int), cudaMemcpyDeviceToHost, st), "fused: flags");
         GC_CUDA(cudaStreamSynchronize(st), "fused: flags");
@@ -2172,9 +2225,13 @@ int passes(GcFused* f, const GcParams& p, int drive, bool hooks) {
 // device too and do nothing, and the host rebuilds the lists and queues the
 // step's passes again (the membrane passes run twice, with the same results).
 // The GPU then does not wait for the host in every step (15 us of a 90 us
-// step of a 6 thousand particle channel).  Steps with outputs written while
-// they run, with profiling marks and with the pair tiles wait for the flag
-// first.
+// step of a 6 thousand particle channel).  From kAheadMost particles on the
+// wait is below 3 % of a step and less than the passes queued twice cost (4.2 M
+// suspension: 4.17 ms a step waiting, 4.22 ahead; 524 k: 601 and 597 us; 350 k
+// sheared suspension: 549 and 532 us); steps with outputs written while they
+// run, with profiling marks and with the pair tiles wait too.
+constexpr int kAheadMost = 600000;
+
 int one_step(GcFused* f, int drive) {
     cudaStream_t st = f->st;
     f->step += 1;
@@ -2183,7 +2240,7 @@ int one_step(GcFused* f, int drive) {
     if (f->ens) GC_TRY(launch_step_begin(f, st));
     else GC_CUDA(cudaMemsetAsync(f->rebuild, 0, sizeof(int), st), "fused: flag");
     GC_TRY(launch_integrate(f, st, p));
-    const bool ahead = f->lists && !f->early && !f->profile;
+    const bool ahead = f->lists && !f->early && !f->profile && f->n < kAheadMost;
     cudaStream_t fs = ahead ? f->fst : st;
     if (ahead) {
         GC_CUDA(cudaEventRecord(f->ev_flag[0], st), "fused: flag");
@@ -2226,10 +2283,7 @@ int launch_rebuild_body(GcFused* f, cudaStream_t st) {
         GC_TRY(tiles_build(f, st, f->a.pos, false));
         return build_morse_lists(f, st, f->mpos, false);
     }
-    float cut = f->p.rc + f->skin;
-    fk_build_list<<<nb, f->block, 0, st>>>(n, f->dsys, f->a.sys, f->a.pos, f->sb.cnt, f->nbr, f->cnt, f->cap,
-                                          cut * cut, f->oflag, f->need, 0);
-    GC_CHECK_LAUNCH("fused: build lists");
+    GC_TRY(launch_build(f, st, f->a.pos, 0));
     return build_morse_lists(f, st, f->mpos, false);
 }
 

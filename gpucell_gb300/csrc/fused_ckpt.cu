@@ -121,13 +121,10 @@ int rebuild_from_ref(GcFused* f) {
                                        "a handle with per-particle lists (GcFusedOptions.tiles = 0)");
         return build_morse_lists_from_ref(f, st);
     }
-    float cut = f->p.rc + f->skin;
     for (int attempt = 0; attempt < 4; ++attempt) {
         GC_CUDA(cudaMemsetAsync(f->oflag, 0, sizeof(unsigned), st), "restore: flags");
         GC_CUDA(cudaMemsetAsync(f->need, 0, sizeof(int), st), "restore: flags");
-        fk_build_list<<<nb, f->block, 0, st>>>(n, f->dsys, f->a.sys, f->refpos, f->sb.cnt, f->nbr, f->cnt, f->cap,
-                                              cut * cut, f->oflag, f->need, 0);
-        GC_CHECK_LAUNCH("restore: build lists");
+        GC_TRY(launch_build(f, st, f->refpos, 0));
         GC_CUDA(cudaMemcpyAsync(&f->h->oflag, f->oflag, sizeof(unsigned), cudaMemcpyDeviceToHost, st), "restore");
         GC_CUDA(cudaMemcpyAsync(&f->h->need, f->need, sizeof(int), cudaMemcpyDeviceToHost, st), "restore");
         GC_CUDA(cudaStreamSynchronize(st), "restore");

@@ -391,6 +391,7 @@ int grown_capacity(const GcFused* f, int at_least);
 int build_grids(GcFused* f);
 int sync_dstep(GcFused* f);
 int rebuild_lists(GcFused* f);
+int launch_build(GcFused* f, cudaStream_t st, const float4* bpos, int walls_only);
 int launch_membranes(GcFused* f, cudaStream_t st, const GcParams& p);
 int build_morse_lists(GcFused* f, cudaStream_t st, const float4* mp, bool host);
 int ensure_early_stream(GcFused* f);
@@ -409,15 +410,6 @@ int store_range(GcFused* f, unsigned id_base, int count, float* pos, float* vel,
 int store_cells_range(GcFused* f, int c0, int nc, int m0, int nv, int t0, int nt, float* area, float* vol,
                       float* defforce, float* aggforce, float* trinordir, float* tricenter, float* pararea,
                       int to_device);
-
-#ifndef GC_BUILD_MIN_BLOCKS
-#define GC_BUILD_MIN_BLOCKS 4   // 64 registers: the build ran 0.554 ms against 0.578 ms unbounded (524k particles)
-#endif
-__global__ void __launch_bounds__(kMaxBS, GC_BUILD_MIN_BLOCKS) fk_build_list(int n, const SysInfo* __restrict__ sys,
-                                                     const int* __restrict__ sysid, const float4* __restrict__ pos,
-                                                     const unsigned* __restrict__ start, int* __restrict__ nbr,
-                                                     int* __restrict__ cnt, int cap, float cut2, unsigned* flags,
-                                                     int* __restrict__ need, int walls_only);
 
 __global__ void fk_gather_mpos(int ncp, const SysInfo* __restrict__ sys, const int* __restrict__ msys,
                                const int* __restrict__ slot_of, const float4* __restrict__ pos,

@@ -624,16 +624,12 @@ int tiles_build(GcFused* f, cudaStream_t st, const float4* bpos, bool host) {
 // rc + skin), for the wall velocity.
 int wall_lists(GcFused* f, cudaStream_t st, const float4* bpos, bool host) {
     if (!any_bound2(f)) return GC_OK;
-    const int n = f->n, nb = gc_blocks(n, f->block);
-    const float cut = f->p.rc + f->skin;
     for (int attempt = 0; attempt < 4; ++attempt) {
         if (host) {
             GC_CUDA(cudaMemsetAsync(f->oflag, 0, sizeof(unsigned), st), "fused: flags");
             GC_CUDA(cudaMemsetAsync(f->need, 0, sizeof(int), st), "fused: flags");
         }
-        fk_build_list<<<nb, f->block, 0, st>>>(n, f->dsys, f->a.sys, bpos, f->sb.cnt, f->nbr, f->cnt, f->cap,
-                                              cut * cut, f->oflag, f->need, 1);
-        GC_CHECK_LAUNCH("fused: wall lists");
+        GC_TRY(launch_build(f, st, bpos, 1));
         if (!host) return GC_OK;
         GC_CUDA(cudaMemcpyAsync(&f->h->oflag, f->oflag, sizeof(unsigned), cudaMemcpyDeviceToHost, st), "fused: flags");
         GC_CUDA(cudaMemcpyAsync(&f->h->need, f->need, sizeof(int), cudaMemcpyDeviceToHost, st), "fused: flags");

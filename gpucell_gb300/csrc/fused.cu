@@ -1380,19 +1380,23 @@ __device__ __forceinline__ void morse_run(const GcParams& p, const GcGrid& g, fl
 // so every pair within MaxCut until then is listed); each step evaluates
 // only the listed pairs.
 //
-// The list build (fk_mlist) runs eight lanes per vertex in aggregation-grid
-// order over the (2R+1)^3 aggregation cubes around it (R = 2 for cubes at
-// least MaxCut/2 wide, 1 for cubes at least MaxCut wide): lane k scans the
-// rows (dy, dz) k, k + 8, ... of the stencil, skipping rows and cubes
-// farther than the cut-off; a first pass counts each lane's candidates, a
-// scan places them, and a second pass writes them, so a vertex's list is
-// lane 0's candidates, then lane 1's, ... in scan order.  The sort is stable
-// and membrane vertices are in id order, so within a cube the candidates
-// ascend by id.  RUNS (every cell is one contiguous id range that carries
-// its CellTab index, checked at set-up): a cube of the own cell alone is
-// skipped from its first and last ids, and otherwise the own cell is one run
-// bounded by two binary searches; without RUNS every candidate's CellTab is
-// compared.  Both find the same candidates in the same order.
+// The list build (fk_mlist) runs a warp per vertex over the (2R+1)^3
+// aggregation cubes around it (R = 2 for cubes at least MaxCut/2 wide, 1 for
+// cubes at least MaxCut wide).  The lanes test 32 cubes at a time (cubes
+// farther than the cut-off are not read) and then go through each cube that
+// is left together, lane k taking the candidates k, k + 32, ...: consecutive
+// loads and no lane waiting for another.  A first pass counts, a scan places
+// the lists, and a second pass writes them in scan order.  It is bound by
+// instruction issue (73 % of the slots, 27 of 32 lanes active): 88 + 106 us
+// at 41 thousand vertices, against 232 + 293 us with eight lanes per vertex
+// that scanned rows of cubes each by itself (9 of 32 lanes active), and
+// 164 + 193 us with eight lanes going through the cubes together (few warps
+// held the vertices with many candidates).  RUNS (every cell is one
+// contiguous id range that carries its CellTab index, checked at set-up): a
+// candidate's id says whether it is of the own cell, and a cube whose first
+// and last ids are is not read (the sort is stable and membrane vertices are
+// in id order, so the ids of a cube ascend).  Without RUNS every candidate's
+// CellTab is compared.  Both find the same candidates in the same order.
 //
 // The pass (fk_maggl) runs eight lanes per vertex in membrane order, lane k
 // taking the entries k, k + 8, ... of the vertex's list; the group adds its
@@ -1412,115 +1416,90 @@ __global__ void __launch_bounds__(kAggBS) fk_mlist(int ncp, GcParams p, float cu
                                                    const unsigned* __restrict__ start,
                                                    const float4* __restrict__ mspos, const int* __restrict__ celltab,
                                                    const int2* __restrict__ cell_verts, unsigned* __restrict__ moff,
-                                                   unsigned* __restrict__ mcnt, int* __restrict__ mlist,
-                                                   unsigned mcap, unsigned* __restrict__ oflag) {
+                                                   int* __restrict__ mlist, unsigned mcap,
+                                                   unsigned* __restrict__ oflag) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int q = (int)(t / kAggLanes), k = (int)(t % kAggLanes);
-    if (q >= ncp) return;   // whole groups: kAggLanes divides the block
+    const int q = (int)(t / 32), k = (int)(t % 32);
+    if (q >= ncp) return;   // whole warps: 32 divides the block
+    if (FILL && moff[ncp] > mcap) {   // the lists do not fit: the host grows them
+        if (k == 0 && q == 0) atomicOr(oflag, kMorseFull);
+        return;
+    }
+    const unsigned below = (1u << k) - 1u;
     const int v = order[q];
     const SysInfo& S = sys[msys ? msys[v] : 0];
     const GcGrid& g = S.mg;
     const float3 xi = xyz(mspos[q]);
     const int ci = celltab[v];
-    unsigned own_lo = 0, own_hi = 0;   // ids of the vertex's own cell
+    unsigned own_lo = 0, own_n = 0;   // ids of the vertex's own cell: own_lo .. own_lo + own_n
     if (RUNS) {
-        int2 cv = cell_verts[ci];
+        const int2 cv = cell_verts[ci];
         own_lo = S.cs + (unsigned)(cv.x - (int)S.m0);
-        own_hi = S.cs + (unsigned)(cv.y - (int)S.m0);
+        own_n = (unsigned)(cv.y - cv.x);
     }
-    const size_t slot = (size_t)v * kAggLanes + k;
-    unsigned w = 0, wend = 0;   // this lane's entries (FILL): after the vertex's offset, the lower lanes' counts
-    bool write = true;
-    if (FILL) {
-        w = moff[v];
-        for (int l = 0; l < k; ++l) w += mcnt[(size_t)v * kAggLanes + l];
-        wend = w + mcnt[slot];
-        if (moff[ncp] > mcap) {   // the lists do not fit: the host grows them
-            write = false;
-            if (k == 0 && q == 0) atomicOr(oflag, kMorseFull);
-        }
-    }
+    unsigned w = FILL ? moff[v] : 0u;   // next entry of the vertex (the same in all lanes)
     const float cut2 = cutl * cutl;
-    unsigned cnt = 0;
-    auto take = [&](unsigned s, float3 d) {
-        const float r2 = norm2_rn(d);
-        if (r2 < cut2) {
-            if (FILL) {
-                if (write && w < wend) mlist[w] = order[s];
-                ++w;
-            } else {
-                ++cnt;
-            }
-        }
-    };
     const int cx = cube_coord(xi.x, 0, g), cy = cube_coord(xi.y, 1, g), cz = cube_coord(xi.z, 2, g);
-    const int R = S.mlr, side = 2 * R + 1;
+    const int R = S.mlr, side = 2 * R + 1, ncube = side * side * side;
     // distance from the vertex to the cube dc steps away along an axis (its
-    // offset f inside its own cube, cube width w): rows and cubes farther
-    // than the cut-off (with a margin far above the rounding) hold no
-    // candidate and are not read
+    // offset f inside its own cube, cube width w): cubes farther than the
+    // cut-off (with a margin far above the rounding) hold no candidate and
+    // are not read
     const float wx = 1.f / g.invw[0], wy = 1.f / g.invw[1], wz = 1.f / g.invw[2];
-    const float fx = xi.x - (g.origin[0] + (float)cx * wx), fy = xi.y - (g.origin[1] + (float)cy * wy),
-                fz = xi.z - (g.origin[2] + (float)cz * wz);
+    auto offset = [&](float x, int c, float w, int axis) {   // of the image inside cube c (x may lie outside the box)
+        const float f = x - (g.origin[axis] + (float)c * w);
+        return g.pmask & (1 << axis) ? f - g.L[axis] * rintf(f / g.L[axis]) : f;
+    };
+    const float fx = offset(xi.x, cx, wx, 0), fy = offset(xi.y, cy, wy, 1), fz = offset(xi.z, cz, wz, 2);
     auto gap = [](int dc, float f, float w) {
         return fmaxf(0.f, dc > 0 ? (float)dc * w - f : (dc < 0 ? f - (float)(dc + 1) * w : 0.f));
     };
     const float cutm = cutl + 1e-3f, cutm2 = cutm * cutm;
-    for (int row = k; row < side * side; row += kAggLanes) {
-        const int dz = row / side - R, dy = row % side - R;
-        const float gz = gap(dz, fz, wz), gy = gap(dy, fy, wy), dyz = gy * gy + gz * gz;
-        if (dyz > cutm2) continue;
-        const int z = cube_step(cz, dz, 2, g);
-        const int y = cube_step(cy, dy, 1, g);
-        if (z < 0 || y < 0) continue;
-        for (int dx = -R; dx <= R; ++dx) {
-            const float gx = gap(dx, fx, wx);
-            if (dyz + gx * gx > cutm2) continue;
-            int x = cube_step(cx, dx, 0, g);
-            if (x < 0) continue;
-            int c = S.mcube0 + cube_key(x, y, z, g);
-            const unsigned s0 = start[c], s1 = start[c + 1];
-            if (s0 == s1) continue;
-            auto run = [&](unsigned a, unsigned b) {
-                for (unsigned s = a; s < b; ++s) take(s, min_image(xi, xyz(mspos[s]), g));
-            };
-            if (RUNS) {
-                const unsigned id_first = fid(mspos[s0]), id_last = fid(mspos[s1 - 1]);
-                if (own_hi < id_first || own_lo > id_last) {
-                    run(s0, s1);
-                    continue;
+    // half the box on periodic axes (the bound of a plain difference), else infinite
+    const float hx = g.pmask & 1 ? g.halfL[0] : INFINITY, hy = g.pmask & 2 ? g.halfL[1] : INFINITY,
+                hz = g.pmask & 4 ? g.halfL[2] : INFINITY;
+    auto image = [](float a, float b, float half, float L) {   // min_image_1
+        const float d = __fsub_rn(a, b);
+        return fabsf(d) > half ? __fsub_rn(d, copysignf(L, d)) : d;
+    };
+    for (int c0 = 0; c0 < ncube; c0 += 32) {
+        // lane k tests cube c0 + k of the stencil
+        unsigned s0 = 0, s1 = 0;
+        const int c = c0 + k;
+        if (c < ncube) {
+            const int dx = c % side - R, dy = c / side % side - R, dz = c / (side * side) - R;
+            const float gx = gap(dx, fx, wx), gy = gap(dy, fy, wy), gz = gap(dz, fz, wz);
+            const int x = cube_step(cx, dx, 0, g), y = cube_step(cy, dy, 1, g), z = cube_step(cz, dz, 2, g);
+            if (x >= 0 && y >= 0 && z >= 0 && gy * gy + gz * gz + gx * gx <= cutm2) {
+                const int key = S.mcube0 + cube_key(x, y, z, g);
+                s0 = start[key];
+                s1 = start[key + 1];
+                // a cube of the own cell alone holds no candidate
+                if (RUNS && s0 < s1 && fid(mspos[s0]) - own_lo <= own_n && fid(mspos[s1 - 1]) - own_lo <= own_n) s1 = s0;
+            }
+        }
+        unsigned left = __ballot_sync(0xffffffffu, s0 < s1);
+        while (left) {
+            const int src = __ffs(left) - 1;
+            left &= left - 1;
+            const unsigned a = __shfl_sync(0xffffffffu, s0, src), b = __shfl_sync(0xffffffffu, s1, src);
+            for (unsigned u = a; u < b; u += 32) {
+                const unsigned s = u + k;
+                bool hit = false;
+                if (s < b) {
+                    const float4 y = mspos[s];
+                    const float3 d = f3(image(xi.x, y.x, hx, g.L[0]), image(xi.y, y.y, hy, g.L[1]),
+                                        image(xi.z, y.z, hz, g.L[2]));
+                    hit = norm2_rn(d) < cut2;
+                    hit = hit && (RUNS ? fid(y) - own_lo > own_n : celltab[order[s]] != ci);
                 }
-                // ids ascend within a cube: a cube of the own cell alone has no candidate
-                if (own_lo <= id_first && id_last <= own_hi) continue;
-                unsigned lo = s0, hi = s1;
-                while (lo < hi) {   // first candidate of the own cell
-                    unsigned mid = (lo + hi) >> 1;
-                    if (fid(mspos[mid]) < own_lo) lo = mid + 1;
-                    else hi = mid;
-                }
-                const unsigned a = lo;
-                hi = s1;
-                while (lo < hi) {   // first candidate past it
-                    unsigned mid = (lo + hi) >> 1;
-                    if (fid(mspos[mid]) <= own_hi) lo = mid + 1;
-                    else hi = mid;
-                }
-                run(s0, a);
-                run(lo, s1);
-            } else {
-                for (unsigned s = s0; s < s1; ++s)
-                    if (celltab[order[s]] != ci) take(s, min_image(xi, xyz(mspos[s]), g));
+                const unsigned m = __ballot_sync(0xffffffffu, hit);
+                if (FILL && hit) mlist[w + __popc(m & below)] = order[s];
+                w += __popc(m);
             }
         }
     }
-    if (!FILL) {
-        // this lane's count, and the vertex's total (the group's eight lanes)
-        mcnt[slot] = cnt;
-        const unsigned gm = 0xFFu << (threadIdx.x & 24);
-#pragma unroll
-        for (int o = kAggLanes / 2; o; o >>= 1) cnt += __shfl_xor_sync(gm, cnt, o, kAggLanes);
-        if (k == 0) moff[v] = cnt;
-    }
+    if (!FILL && k == 0) moff[v] = w;
 }
 
 __global__ void __launch_bounds__(kAggBS) fk_maggl(int ncp, GcParams p, const SysInfo* __restrict__ sys,
@@ -1802,7 +1781,7 @@ int ensure_agg_sort_bufs(GcFused* f) {
 }
 
 // The Morse lists of the current membrane positions `mp` (membrane order):
-// sort the vertices into the aggregation cubes, count each lane's
+// sort the vertices into the aggregation cubes, count each vertex's
 // candidates within MaxCut + skin, scan, write.  From the host (`host`) the
 // entries grow to fit, with room for the rebuilds of captured steps; inside
 // a captured step a list that does not fit raises kMorseFull in the
@@ -1813,7 +1792,6 @@ int build_morse_lists(GcFused* f, cudaStream_t st, const float4* mp, bool host) 
     const size_t nl = (size_t)ncp + 1;   // per vertex, scanned into offsets
     if (host && !f->moff) {
         GC_CUDA(cudaMalloc(&f->moff, nl * sizeof(unsigned)), "fused: Morse lists");
-        GC_CUDA(cudaMalloc(&f->mcnt, (size_t)ncp * kAggLanes * sizeof(unsigned)), "fused: Morse lists");
         GC_CUDA(cudaMalloc(&f->mscan, gc_scan_blocks((int)nl) * sizeof(unsigned)), "fused: Morse lists");
         drop_graphs(f);
     }
@@ -1824,17 +1802,17 @@ int build_morse_lists(GcFused* f, cudaStream_t st, const float4* mp, bool host) 
     fk_msort<<<gc_blocks(ncp, f->block), f->block, 0, st>>>(ncp, f->mvals, mp, f->parea, f->mspos, f->msarea);
     GC_CHECK_LAUNCH("fused: aggregation order");
     const float cutl = f->p.maxcut + f->skin;
-    const int nba = gc_blocks((int)((long long)ncp * kAggLanes), kAggBS);
+    const int nba = gc_blocks((long long)ncp * 32, kAggBS);
     GC_CUDA(cudaMemsetAsync(f->moff + (nl - 1), 0, sizeof(unsigned), st), "fused: Morse lists");
     auto pass = [&](auto fill) -> int {
         constexpr bool F = decltype(fill)::value;
         if (f->agg_runs)
-            fk_mlist<true, F><<<nba, kAggBS, 0, st>>>(ncp, f->p, cutl, f->dsys, f->msys, f->mvals, f->sb_agg.cnt,
-                                                      f->mspos, f->celltab, f->cell_verts, f->moff, f->mcnt,
+            fk_mlist<true, F><<<nba, kAggBS, 0, st>>>(ncp, f->p, cutl, f->dsys, f->msys, f->mvals,
+                                                      f->sb_agg.cnt, f->mspos, f->celltab, f->cell_verts, f->moff,
                                                       f->mlist, (unsigned)f->mcap, f->oflag);
         else
-            fk_mlist<false, F><<<nba, kAggBS, 0, st>>>(ncp, f->p, cutl, f->dsys, f->msys, f->mvals, f->sb_agg.cnt,
-                                                       f->mspos, f->celltab, f->cell_verts, f->moff, f->mcnt,
+            fk_mlist<false, F><<<nba, kAggBS, 0, st>>>(ncp, f->p, cutl, f->dsys, f->msys, f->mvals,
+                                                       f->sb_agg.cnt, f->mspos, f->celltab, f->cell_verts, f->moff,
                                                        f->mlist, (unsigned)f->mcap, f->oflag);
         GC_CHECK_LAUNCH("fused: Morse lists");
         return GC_OK;
@@ -3537,7 +3515,7 @@ int gc_fused_destroy(GcFused* f) {
     for (int c = 0; c < 4; ++c)
         if (f->xev[c]) cudaEventDestroy(f->xev[c]);
     if (f->sortmem_agg) cudaFree(f->sortmem_agg);
-    for (void* q : {(void*)f->moff, (void*)f->mcnt, (void*)f->mscan, (void*)f->mlist, (void*)f->mref})
+    for (void* q : {(void*)f->moff, (void*)f->mscan, (void*)f->mlist, (void*)f->mref})
         if (q) cudaFree(q);
     if (f->xst) cudaStreamSynchronize(f->xst);
     for (int k = 0; k < 4; ++k)

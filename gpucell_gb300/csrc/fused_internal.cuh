@@ -277,11 +277,9 @@ struct GcFused {
     void* sortmem_agg = nullptr;   // the aggregation sort's own temporaries (the Morse list build)
     int sort_agg_n = 0, sort_agg_K = 0;
     // Morse Verlet lists: per vertex the offset of its entries (ncp + 1,
-    // scanned from the counts), per vertex and lane of the build the count,
-    // the scan's block sums, the entries (membrane indices) and their
-    // capacity, and the membrane positions of a restore
+    // scanned from the counts), the scan's block sums, the entries (membrane
+    // indices) and their capacity, and the membrane positions of a restore
     unsigned* moff = nullptr;
-    unsigned* mcnt = nullptr;
     unsigned* mscan = nullptr;
     int* mlist = nullptr;
     size_t mcap = 0;

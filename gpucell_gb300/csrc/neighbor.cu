@@ -11,7 +11,7 @@
 // The array sort then restores d_sortpart to ids.
 //
 // The sort is a stable counting sort by cube: a warp-aggregated count, one
-// device-wide exclusive scan of the cube counts, a scatter, and a per-cube
+// device-wide exclusive scan of the cube counts, a scatter, and a
 // rank fix that restores the input order inside each cube.  The result is
 // exactly that of a stable radix sort, with one pass over the keys instead of
 // one per digit.
@@ -79,42 +79,30 @@ __global__ void k_sort_scatter(int n, int K, const int* __restrict__ keys, const
     osrc[d] = i;
 }
 
-// One warp per cube: the final position of each element inside its cube is
-// the number of elements of that cube that came earlier in the input.
-__global__ void k_sort_fix(int K, const unsigned* __restrict__ start, const int* __restrict__ tkey,
+// One thread per element: its final position inside its cube is the number of
+// elements of that cube that came earlier in the input.  Bound by the launch
+// and by memory: a cube of the fused step's lists holds 3 elements and one of
+// the boundary's 27, so a warp per cube left most lanes idle (4.2 M
+// particles: 167 us then, 30 now; 1 M on the boundary: 14.6 and 12.9).
+__global__ void k_sort_fix(int n, const unsigned* __restrict__ start, const int* __restrict__ tkey,
                            const int* __restrict__ tval, const int* __restrict__ tsrc, int* __restrict__ keys,
                            int* __restrict__ vals) {
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (warp >= K) return;
-    unsigned b = start[warp], e = start[warp + 1];
-    unsigned c = e - b;
-    if (c == 0) return;
-    if (c <= 32) {
-        int src = lane < (int)c ? tsrc[b + lane] : 0x7fffffff;
-        int r = 0;
-        for (int t = 0; t < (int)c; ++t) {
-            int o = __shfl_sync(0xffffffffu, src, t);
-            r += (o < src);
-        }
-        if (lane < (int)c) {
-            keys[b + r] = tkey[b + lane];
-            vals[b + r] = tval[b + lane];
-        }
-    } else {
-        for (unsigned q = lane; q < c; q += 32) {
-            int src = tsrc[b + q];
-            unsigned r = 0;
-            for (unsigned t = 0; t < c; ++t) r += (tsrc[b + t] < src);
-            keys[b + r] = tkey[b + q];
-            vals[b + r] = tval[b + q];
-        }
-    }
+    const int d = blockIdx.x * blockDim.x + threadIdx.x;
+    if (d >= n) return;
+    const int k = tkey[d], src = tsrc[d], val = tval[d];
+    const unsigned b = start[k], e = start[k + 1];
+    unsigned r = b;
+#pragma unroll 4
+    for (unsigned t = b; t < e; ++t) r += tsrc[t] < src;
+    keys[r] = k;
+    vals[r] = val;
 }
 
 // --------------------------------------------------------------------------
-// Device-wide exclusive scan of uint32 (two levels: 4096 per block, block
-// sums scanned by one block).  Writes out[0..n] with out[n] = total.
+// Device-wide exclusive scan of uint32 (two levels: 4096 per block, whose
+// sums each block of the second launch adds up for itself: a third launch that
+// scanned them cost as much as the others, 3 us, at every size measured; one
+// tile needs one launch).  Writes out[0..n] with out[n] = total.
 // --------------------------------------------------------------------------
 constexpr int kScanBS = 1024, kScanIPT = 4, kScanTile = kScanBS * kScanIPT;
 
@@ -147,7 +135,7 @@ __device__ unsigned block_exclusive_scan(unsigned v, unsigned* sh, unsigned* tot
 __global__ void k_scan_tiles(int n, const unsigned* in, unsigned* out,  // may alias (in-place scan)
                              unsigned* __restrict__ bsum) {
     __shared__ unsigned sh[32];
-    long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanIPT;
+    const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanIPT;
     unsigned v[kScanIPT], s = 0;
 #pragma unroll
     for (int k = 0; k < kScanIPT; ++k) {
@@ -161,31 +149,22 @@ __global__ void k_scan_tiles(int n, const unsigned* in, unsigned* out,  // may a
         if (base + k < n) out[base + k] = off;
         off += v[k];
     }
-    if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
+    if (threadIdx.x != 0) return;
+    bsum[blockIdx.x] = tot;
+    if (gridDim.x == 1) out[n] = tot;
 }
 
-__global__ void k_scan_bsums(int nb, unsigned* __restrict__ bsum, unsigned* __restrict__ total_out) {
-    __shared__ unsigned sh[32];
-    unsigned v[kScanIPT], s = 0;
-    int base = threadIdx.x * kScanIPT;
-#pragma unroll
-    for (int k = 0; k < kScanIPT; ++k) {
-        v[k] = (base + k < nb) ? bsum[base + k] : 0u;
-        s += v[k];
-    }
-    unsigned tot;
-    unsigned off = block_exclusive_scan(s, sh, &tot);
-#pragma unroll
-    for (int k = 0; k < kScanIPT; ++k) {
-        if (base + k < nb) bsum[base + k] = off;
-        off += v[k];
-    }
-    if (threadIdx.x == 0) *total_out = tot;
-}
-
+// Adds the sums of the tiles before it to every tile.
 __global__ void k_scan_add(int n, unsigned* __restrict__ out, const unsigned* __restrict__ bsum) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] += bsum[i / kScanTile];
+    __shared__ unsigned sh[32];
+    unsigned s = 0, tot;
+    for (int t = threadIdx.x; t < (int)blockIdx.x; t += kScanBS) s += bsum[t];
+    block_exclusive_scan(s, sh, &tot);
+    const long long base = (long long)blockIdx.x * kScanTile + threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < kScanIPT; ++k)
+        if (base + k * kScanBS < n) out[base + k * kScanBS] += tot;
+    if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) out[n] = tot + bsum[blockIdx.x];
 }
 
 __global__ void k_maxkey(int n, const int* __restrict__ keys, int* __restrict__ out) {
@@ -242,6 +221,36 @@ __global__ void k_gather(int n, int* __restrict__ sortpart, const int* __restric
     }
 }
 
+// The gathered arrays back to the caller's, in one launch (blockIdx.y: which)
+// instead of a copy each, whose gaps cost more than the bytes below a million
+// particles.  The sources lie on 16-byte boundaries; a caller's array that
+// does not is written by words.
+struct CopyBack {
+    static constexpr int kMost = 7;
+    unsigned* dst[kMost];
+    const unsigned* src[kMost];
+    size_t words[kMost];
+    int count = 0;
+    void add(void* d, const void* s, size_t w) {
+        dst[count] = (unsigned*)d;
+        src[count] = (const unsigned*)s;
+        words[count++] = w;
+    }
+};
+
+__global__ void k_copy_back(CopyBack c) {
+    unsigned* __restrict__ d = c.dst[blockIdx.y];
+    const unsigned* __restrict__ s = c.src[blockIdx.y];
+    const size_t w = c.words[blockIdx.y], i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    size_t quads = 0;
+    if (((size_t)d & 15) == 0) {
+        quads = w / 4;
+        for (size_t i = i0; i < quads; i += step) ((uint4*)d)[i] = ((const uint4*)s)[i];
+    }
+    for (size_t i = 4 * quads + i0; i < w; i += step) d[i] = s[i];
+}
+
 // In-place exclusive scan of buf[0..n) with buf[n] = total; `bsum` holds
 // (n / kScanTile + 1) block sums.
 int scan_exclusive_with(unsigned* buf, int n, unsigned* bsum, cudaStream_t st) {
@@ -249,9 +258,8 @@ int scan_exclusive_with(unsigned* buf, int n, unsigned* bsum, cudaStream_t st) {
     if (nb > kScanTile) return gc_fail(GC_EINVAL, "scan of %d elements exceeds the two-level limit", n);
     k_scan_tiles<<<nb, kScanBS, 0, st>>>(n, buf, buf, bsum);
     GC_CHECK_LAUNCH("scan: tiles");
-    k_scan_bsums<<<1, kScanBS, 0, st>>>(nb, bsum, buf + n);
-    GC_CHECK_LAUNCH("scan: block sums");
-    k_scan_add<<<gc_blocks(n, kBS), kBS, 0, st>>>(n, buf, bsum);
+    if (nb == 1) return GC_OK;
+    k_scan_add<<<nb, kScanBS, 0, st>>>(n, buf, bsum);
     GC_CHECK_LAUNCH("scan: add");
     return GC_OK;
 }
@@ -265,7 +273,7 @@ int sort_with(int n, int K, int* keys, int* vals, const GcSortBufs& b, unsigned*
     GC_TRY(scan_exclusive_with(b.cnt, K, b.bsum, st));
     k_sort_scatter<<<gc_blocks(n, kBS), kBS, 0, st>>>(n, K, keys, vals, b.cnt, b.rank, b.tkey, b.tval, b.tsrc);
     GC_CHECK_LAUNCH("sort: scatter");
-    k_sort_fix<<<gc_blocks((long long)K * 32, kBS), kBS, 0, st>>>(K, b.cnt, b.tkey, b.tval, b.tsrc, keys, vals);
+    k_sort_fix<<<gc_blocks(n, kBS), kBS, 0, st>>>(n, b.cnt, b.tkey, b.tval, b.tsrc, keys, vals);
     GC_CHECK_LAUNCH("sort: fix");
     return GC_OK;
 }
@@ -409,14 +417,17 @@ static int sort_arrays(int n, int* d_sortpart, int* d_oldpos, int* d_curpos, flo
     GC_CHECK_LAUNCH("SortArrays: gather");
     // The caller's pointers are fixed (src/Particle.cu:575-589), so the
     // gathered arrays are copied back.
-    GC_CUDA(cudaMemcpyAsync(d_totalcoor, o.coor, 12 * (size_t)n, cudaMemcpyDeviceToDevice, s.stream), "copy back");
-    GC_CUDA(cudaMemcpyAsync(d_cc, o.cc, 12 * (size_t)n, cudaMemcpyDeviceToDevice, s.stream), "copy back");
-    GC_CUDA(cudaMemcpyAsync(d_velrhop, o.velrhop, 16 * (size_t)n, cudaMemcpyDeviceToDevice, s.stream), "copy back");
-    GC_CUDA(cudaMemcpyAsync(d_velhalf, o.velhalf, 12 * (size_t)n, cudaMemcpyDeviceToDevice, s.stream), "copy back");
-    GC_CUDA(cudaMemcpyAsync(d_totalforce, o.force, 12 * (size_t)n, cudaMemcpyDeviceToDevice, s.stream), "copy back");
-    GC_CUDA(cudaMemcpyAsync(d_press, o.press, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s.stream), "copy back");
-    if (d_nthro)
-        GC_CUDA(cudaMemcpyAsync(d_nthro, o.nthro, 12 * (size_t)n, cudaMemcpyDeviceToDevice, s.stream), "copy back");
+    CopyBack c;
+    const size_t m = n;
+    c.add(d_totalcoor, o.coor, 3 * m);
+    c.add(d_cc, o.cc, 3 * m);
+    c.add(d_velrhop, o.velrhop, 4 * m);
+    c.add(d_velhalf, o.velhalf, 3 * m);
+    c.add(d_totalforce, o.force, 3 * m);
+    c.add(d_press, o.press, m);
+    if (d_nthro) c.add(d_nthro, o.nthro, 3 * m);
+    k_copy_back<<<dim3(gc_blocks(n, kBS), c.count), kBS, 0, s.stream>>>(c);
+    GC_CHECK_LAUNCH("SortArrays: copy back");
     return GC_OK;
 }
 

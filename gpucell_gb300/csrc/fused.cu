@@ -6,7 +6,9 @@
 //
 //   * State lives in the library, in slot order (sorted by cube), as float4
 //     records: position + global id, velocity, predicted velocity, VelHalf,
-//     force, and (1/d, P/d^2) per particle.  Membrane vertices additionally
+//     force, and (1/d, P/d^2) per particle, and a 32-byte record per slot
+//     that the density pass writes and the force pass gathers (position, id,
+//     predicted velocity, 1/d).  Membrane vertices additionally
 //     have a membrane-ordered copy of their position and crossing counts, so
 //     the membrane kernels index topology directly.
 //   * An ensemble of independent simulations ("systems") shares the arrays.
@@ -368,7 +370,9 @@ __device__ __forceinline__ int scan_rows(int r0, int r1, int k, int i, float3 xi
             else if (x >= g.n[0]) { if (!(g.pmask & 1)) continue; x -= g.n[0]; sx = -g.L[0]; }
             const unsigned jb = start[row + x], je = start[row + (whole ? b : x) + 1];
             const float3 xs = f3(xi.x + sx, xi.y + sy, xi.z + sz);
-            if (mobile_only || (dy == 0 && dz == 0) || k + (int)(je - jb) > cap)
+            // (slot i may lie in another row than its own: it was sorted by the
+            // position before the wrap, which rounds)
+            if (mobile_only || (unsigned)i - jb < je - jb || k + (int)(je - jb) > cap)
                 scan_range<WRITE, true>(pos, jb, je, xs, i, cut2, mobile_only, fl, cap, lst, k);
             else
                 scan_range<WRITE, false>(pos, jb, je, xs, i, cut2, false, 0u, cap, lst, k);

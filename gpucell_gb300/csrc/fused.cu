@@ -8,7 +8,7 @@
 //     records: position + global id, velocity, predicted velocity, VelHalf,
 //     force, and (1/d, P/d^2) per particle, and a 32-byte record per slot
 //     that the density pass writes and the force pass gathers (position, id,
-//     predicted velocity, 1/d).  Membrane vertices additionally
+//     predicted velocity, 1/d less its value at rest).  Membrane vertices additionally
 //     have a membrane-ordered copy of their position and crossing counts, so
 //     the membrane kernels index topology directly.
 //   * An ensemble of independent simulations ("systems") shares the arrays.
@@ -542,7 +542,7 @@ __device__ __forceinline__ void wall_velocity(int q, int nwall, int n, const GcP
     const float3 r = den > 0.f ? f3(2.f * w4.x - num.x / den, 2.f * w4.y - num.y / den, 2.f * w4.z - num.z / den)
                                : f3(w4.x, w4.y, w4.z);
     v[i] = make_float4(r.x, r.y, r.z, 0.f);
-    if (rec) rec[i] = PairRec{pos[i], make_float4(r.x, r.y, r.z, p.mass / p.rho0)};
+    if (rec) rec[i] = PairRec{pos[i], make_float4(r.x, r.y, r.z, 0.f)};
 }
 
 template <bool ENS>
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
     if (t != PT_FLUID && t != PT_MEMB) {
         if (s == 0) {
             dp[i] = make_float2(p.mass / p.rho0, 0.f);
-            if (t == PT_B1) rec[i] = PairRec{xi4, make_float4(0.f, 0.f, 0.f, p.mass / p.rho0)};
+            if (t == PT_B1) rec[i] = PairRec{xi4, make_float4(0.f, 0.f, 0.f, 0.f)};
         }
         return;
     }
@@ -669,7 +669,9 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
     float inv_d = __frcp_rn(sum);
     dp[i] = make_float2(inv_d, c2 * (rho - p.rho0) * inv_d * inv_d);
     const float4 vp = vpred[i];
-    rec[i] = PairRec{xi4, make_float4(vp.x, vp.y, vp.z, inv_d)};
+    // 1/d - 1/d0 from the difference of the densities, which is exact where they are close
+    const float z = p.rho0 > 0.f ? (p.rho0 - rho) * inv_d / p.rho0 : inv_d;
+    rec[i] = PairRec{xi4, make_float4(vp.x, vp.y, vp.z, z)};
 }
 
 // ---------------------------------------------------------------------------
@@ -751,16 +753,20 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
     // derives it, in a captured step at each replay)
     const uint32_t key = !NOISE || KEYS ? 0u : nkey[s];
     const float4 vi = ri.v;
-    // P/d^2 of a particle from w = 1/d and its squared sound speed:
-    // c^2 (rho - rho0) / d^2 = c^2 w (m - rho0 w), zero at rho0 (walls) to a
-    // rounding.  Three operations instead of a second gather per pair, which
-    // took a fifth of the pass's L1 wavefronts.  Where all sound speeds are
+    // P/d^2 of a particle from z = 1/d - 1/d0 (d0 = rho0/m) and its squared
+    // sound speed: c^2 (rho - rho0) / d^2 = -c^2 rho0 z / d, zero at rho0
+    // (walls).  Four operations instead of a second gather per pair, which
+    // took a fifth of the pass's L1 wavefronts; from 1/d itself it is c^2
+    // (m - rho0/d) / d, whose difference loses the digits that z keeps (the
+    // force from given densities was 1.0e-6 off in the median instead of
+    // 2.6e-7).  Without a rest density z is 1/d.  Where all sound speeds are
     // one, B1 is false or c1sq = c2sq.
-    auto pterm = [&](float w, unsigned pid) -> float {
+    auto pterm = [&](float z, float inv_d, unsigned pid) -> float {
         const float c2 = B1 ? (pid >= S.cs ? p.c2sq : p.c1sq) : p.c1sq;
-        return (c2 * w) * fmaf(-p.rho0, w, p.mass);
+        return (c2 * inv_d) * fmaf(-p.rho0, z, p.rest_m);
     };
-    const float pti = pterm(ri.v.w, id);
+    const float idi = p.rest_invd + vi.w;   // 1/d
+    const float pti = pterm(vi.w, idi, id);
     float2 fxy = make_float2(0.f, 0.f);
     float fz = 0.f;
     const int call = cnt[i];
@@ -842,9 +848,10 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
         const float F = wendland_f(r2 * inv_r, p);
         const float2 vxy = __ffma2_rn(make_float2(rj.v.x, rj.v.y), make_float2(-1.f, -1.f), make_float2(vi.x, vi.y));
         const float vz = vi.z - rj.v.z;
-        const float fdd = F * (vi.w * rj.v.w);
+        const float idd = p.rest_invd + rj.v.w;
+        const float fdd = F * (idi * idd);
         const float dv = fmaf(dxy.x, vxy.x, fmaf(dxy.y, vxy.y, dz * vz));
-        float cd = (pti + pterm(rj.v.w, idj)) * F - (fdd * p.visB) * dv * ir2;
+        float cd = (pti + pterm(rj.v.w, idd, idj)) * F - (fdd * p.visB) * dv * ir2;
         add_f(-fdd * p.visA, vxy, vz);
         if constexpr (NOISE) {
             // (a pair at the cut-off can give F a rounding-sized negative value: its noise is as small)

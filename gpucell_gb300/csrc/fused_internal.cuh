@@ -156,11 +156,11 @@ struct SlotArrays {
 };
 
 // What the force pass gathers of a neighbour, written by the density pass:
-// position and id, predicted velocity and 1/d in one 32-byte record, which
-// one 256-bit load brings in.
+// position and id, predicted velocity and 1/d (less its value at the rest
+// density) in one 32-byte record, which one 256-bit load brings in.
 struct __align__(32) PairRec {
     float4 x;   // position, id bits
-    float4 v;   // predicted velocity, 1/d
+    float4 v;   // predicted velocity, 1/d - 1/d0
 };
 
 // Membrane topology of one system as given (local, 1-based), until set-up.

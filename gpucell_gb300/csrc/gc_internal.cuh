@@ -61,6 +61,9 @@ struct GcParams {
     float visB;                      // 5 (zeta + eta/3)
     float sqrtA, sqrtAB;             // sqrt(visA), sqrt(visA + visB)
     float noise_pref;                // 2 kT / dt (0 when the noise is off)
+    // 1/d at the rest density and the mass it leaves out of m - rho0/d: m/rho0
+    // and 0, or 0 and m without a rest density
+    float rest_invd, rest_m;
     // Bound1 repulsion (Monaghan 1994, exponents 12 and 4)
     float rep_r0, rep_r0sq, rep_D;
     // Morse aggregation

@@ -163,6 +163,8 @@ int gc_params_from(const Structconst& c, int noise_on, GcParams* p) {
     p->c1sq = c.SoundSpeed1 * c.SoundSpeed1;
     p->c2sq = c.SoundSpeed2 * c.SoundSpeed2;
     p->rho0 = c.DenInit;
+    p->rest_invd = c.DenInit > 0.f ? c.Mass / c.DenInit : 0.f;
+    p->rest_m = c.DenInit > 0.f ? 0.f : c.Mass;
     p->lambda = c.VVsigma;
     p->dt = c.TimeStep;
     p->gx = c.ConstExtForce;

@@ -303,15 +303,18 @@ TILE_PARTIAL_BYTES = {"force": 2 * 14 * 12, "density": 2 * 14 * 4}
 # on the 524,288-particle suspension (warp instructions and FP32 operations
 # per particle; skin 0.125 rc, mean list 166.5), and
 #   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum --clock-control none
-#       -k regex:"fk_(force|density|build_list|mgather|medge|mgeo|mtri|integrate)" -s 8 -c 8 python bench.py
+#       -k regex:"fk_(force|density|build_list|mgather|mgeo_edge|mtri|integrate)" -s 8 -c 8 python bench.py
 #       --no-ensemble --cpu-steps 0 --no-plain --no-engine --no-output --no-parity --no-configs --no-variants
 #       --steps 4 --warmup 3 --profile-steps 1 --e2e-steps 1
-# at full size (DRAM bytes of one launch, one pass).
+# at full size (DRAM bytes of one launch, one pass).  The FP32 operations were
+# counted on the form without packed instructions, which do the same two at a
+# time.
 FORCE_COUNTERS = {
-    "kernel_version": "fk_force<1,0,0,1,0>: one thread per particle over its compact list of acting entries, "
-                      "pair terms as three coefficient vectors, noise and wall-free forms as template switches",
-    "dram_bytes_per_launch_4M": 3.256612864e9 + 0.129022976e9,
-    "warp_inst_per_particle": 278141655 / 524288,
+    "kernel_version": "fk_force<1,0,0,1,0,1,1>: one thread per particle over its compact list of acting entries, "
+                      "32-byte neighbour records, packed FP32 pair terms, noise and wall-free forms as template "
+                      "switches",
+    "dram_bytes_per_launch_4M": 3.215104256e9 + 0.127953920e9,
+    "warp_inst_per_particle": 245566966 / 524288,
     "fp32_flop_per_particle": 4.1227e9 / 524288,
 }
 # SM schedulers of a GB300 (152 SMs x 4, one warp instruction per cycle

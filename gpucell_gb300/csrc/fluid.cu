@@ -76,26 +76,29 @@ __global__ void k_periodic(int n, GcParams p, const int* __restrict__ sortpart, 
     nthro[i] = t;
 }
 
-// K8 -- kernel-sum density of fluid and membrane particles (the particle's
-// own share W(0) comes with its own entry among the candidates).
+// K8 -- kernel-sum density of fluid and membrane particles.
 struct DensityOp {
     float4* velrhop;
     static constexpr int kBlocks = 8;   // resident blocks the registers are cut to
-    static constexpr bool kExact = false;
     struct Extra {};
-    struct Self {};
+    struct Self { unsigned id; };
     struct Acc { float sum; };
     __device__ float cut2(const GcParams& p) const { return p.rc2; }
     __device__ bool active(unsigned id, const GcParams& p) const { return is_mobile(id, p); }
     __device__ bool keep(unsigned id, const GcParams& p) const { return is_sdpd(id, p); }
     __device__ void idle(int) const {}
-    __device__ void begin(Acc& a, Self&, int, unsigned, bool, const GcParams&) const { a.sum = 0.f; }
+    __device__ void begin(Acc& a, Self& s, int, unsigned id, bool, const GcParams&) const {
+        a.sum = 0.f;
+        s.id = id;
+    }
     __device__ void stage(Extra&, int, int, const GcParams&) const {}
-    __device__ void pair(Acc& a, const Self&, const Extra&, int, unsigned, float3, float r2, const GcParams& p) const {
-        a.sum += wendland_w(r2 < kTiny ? 0.f : r2 * rsqrt_ftz(r2), p);
+    __device__ void pair(Acc& a, const Self& s, const Extra&, int, unsigned idj, float3, float r2, const GcParams& p) const {
+        if (idj != s.id) a.sum += wendland_w(r2 < kTiny ? 0.f : r2 * rsqrt_ftz(r2), p);
     }
     __device__ void reduce(Acc& a) const { a.sum = gcsweep::lane_sum(a.sum); }
-    __device__ void finish(const Acc& a, const Self&, int i, const GcParams& p) const { velrhop[i].w = p.mass * a.sum; }
+    __device__ void finish(const Acc& a, const Self&, int i, const GcParams& p) const {
+        velrhop[i].w = p.mass * (p.w0 + a.sum);
+    }
 };
 
 // K9 -- predictor: VelHalf = v + dt/2 F/m, v <- v + lambda dt F/m.
@@ -119,7 +122,6 @@ struct Bound2VelOp {
     float4* velrhop;
     const float3* velhalf;
     static constexpr int kBlocks = 6;   // resident blocks the registers are cut to
-    static constexpr bool kExact = false;
     struct Extra { float3 v[gcsweep::kCap]; };
     struct Self {};
     struct Acc { float3 num; float den; };
@@ -183,7 +185,6 @@ struct SdpdOp {
     const float* press;
     float3* force;
     static constexpr int kBlocks = 6;   // resident blocks the registers are cut to
-    static constexpr bool kExact = false;
     struct Extra { float4 v[gcsweep::kCap]; float pt[gcsweep::kCap]; };
     struct Self { float3 v; float inv_d, pt; unsigned id; };
     struct Acc { float3 f; };
@@ -209,7 +210,7 @@ struct SdpdOp {
     }
     __device__ void pair(Acc& a, const Self& s, const Extra& e, int q, unsigned idj, float3 d, float r2,
                          const GcParams& p) const {
-        if (r2 < kTiny) return;   // the particle itself; coincident particles exert no force
+        if (r2 < kTiny || idj == s.id) return;   // coincident particles exert no force
         const float4 vj = e.v[q];
         const float inv_r = rsqrt_ftz(r2), ir2 = inv_r * inv_r;
         const float F = wendland_f(r2 * inv_r, p);
@@ -238,7 +239,6 @@ struct SdpdOp {
 struct RepulsionOp {
     float3* force;
     static constexpr int kBlocks = 8;   // resident blocks the registers are cut to
-    static constexpr bool kExact = false;
     struct Extra {};
     struct Self {};
     struct Acc { float3 f; };
@@ -302,18 +302,16 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
     return z ^ (z >> 31);
 }
 
-// Number and id checksum of every slot's neighbours.  The sweep marks with a
-// slightly larger cut-off and the pair function applies the predicate of the
-// oracle, bit for bit.
+// Number and id checksum of every slot's neighbours: the pairs that the other
+// sweeps evaluate.
 struct NeighborOp {
     int* count;
     unsigned long long* hash;
     static constexpr int kBlocks = 8;   // resident blocks the registers are cut to
-    static constexpr bool kExact = true;
     struct Extra {};
     struct Self { unsigned id; };
     struct Acc { int cnt; unsigned long long h; };
-    __device__ float cut2(const GcParams& p) const { return p.rc2 * 1.00001f; }
+    __device__ float cut2(const GcParams& p) const { return p.rc2; }
     __device__ bool active(unsigned, const GcParams&) const { return true; }
     __device__ bool keep(unsigned, const GcParams&) const { return true; }
     __device__ void idle(int) const {}
@@ -323,8 +321,8 @@ struct NeighborOp {
         s.id = id;
     }
     __device__ void stage(Extra&, int, int, const GcParams&) const {}
-    __device__ void pair(Acc& a, const Self& s, const Extra&, int, unsigned idj, float3, float r2, const GcParams& p) const {
-        if (r2 >= p.rc2 || idj == s.id) return;
+    __device__ void pair(Acc& a, const Self& s, const Extra&, int, unsigned idj, float3, float, const GcParams&) const {
+        if (idj == s.id) return;
         ++a.cnt;
         a.h += mix64((unsigned long long)idj);
     }

@@ -55,15 +55,11 @@ struct Shared {
     float4 x[kCap];                      // position, id bits
     unsigned mark[2][kWords * kBlock];   // per particle of the group: word w of thread t at w * kBlock + t
     int beg[27], off[28];                // first slot of each cube of the stencil, their scanned sizes
-    float3 shift[27];                    // what brings each cube next to the centre
 };
 
-// First slots, scanned sizes (sh.off[27] is the number of candidates) and
-// shifts of the 27 cubes around cube c.  Cubes beyond a wall axis are empty;
-// periodic axes have at least three cubes, so none is taken twice.  A
-// stencil that crosses a periodic face is brought together below the lower
-// face: what lies at the upper face moves down by the box length, which is
-// exact in FP32 where the minimum image of the difference is not.
+// First slots and scanned sizes (sh.off[27] is the number of candidates) of
+// the 27 cubes around cube c.  Cubes beyond a wall axis are empty; periodic
+// axes have at least three cubes, so none is taken twice.
 __device__ __forceinline__ void stencil(const GcGrid& g, int3 c, const int2* __restrict__ bec, Shared& sh) {
     if (threadIdx.x < 32) {
         const int t = threadIdx.x;
@@ -76,12 +72,6 @@ __device__ __forceinline__ void stencil(const GcGrid& g, int3 c, const int2* __r
                 b = be.x;
                 cnt = max(be.y - be.x, 0);
             }
-            auto down = [&](int cc, int q, int a) {
-                if (!(g.pmask & (1 << a))) return 0.f;
-                const int last = g.n[a] - 1;
-                return (cc == 0 && q == last) || (cc == last && q != 0) ? -g.L[a] : 0.f;
-            };
-            sh.shift[t] = f3(down(c.x, x, 0), down(c.y, y, 1), down(c.z, z, 2));
         }
         int sum = cnt;
 #pragma unroll
@@ -98,13 +88,54 @@ __device__ __forceinline__ void stencil(const GcGrid& g, int3 c, const int2* __r
     __syncthreads();
 }
 
-// Whether x lies outside the box on a periodic axis, or is no number.
-__device__ __forceinline__ bool outside(float3 x, const GcGrid& g) {
-    bool o = !(x.x == x.x && x.y == x.y && x.z == x.z);
-    if (g.pmask & 1) o |= !(x.x >= g.lo[0] && x.x < g.hi[0]);
-    if (g.pmask & 2) o |= !(x.y >= g.lo[1] && x.y < g.hi[1]);
-    if (g.pmask & 4) o |= !(x.z >= g.lo[2] && x.z < g.hi[2]);
-    return o;
+// How the candidates of a cube are tested: bits 1, 2, 4 for the image along
+// x, y, z, or kAny.  kAny also takes positions that are no numbers: a NaN
+// distance counts as within, as in the oracle's test, so that a lost particle
+// shows in its neighbours.
+constexpr int kAny = 8;
+
+// The positions for which the plain difference along an axis decides as the
+// minimum image does: of the cube's own particles within A of the cube's
+// centre, of the candidates within B, where A + B = L - rc.  (A pair more
+// than L/2 apart is then farther than rc either way.)  Particles in the cube
+// they were sorted into keep to that with (L - rc - 2 w) / 2 to spare, w the
+// cube's width, at least 3e-5 rc.  It is tested on the positions: one that
+// the caller has moved since, that lies outside the box, or whose cube came
+// out on the other side of a face by rounding makes its block take images.
+// No limit along wall axes and where the stencil crosses a face (those take
+// the image in any case).
+struct Limits {
+    float3 centre, own, cand;
+    int cross;   // periodic axes along which the stencil crosses a face
+};
+
+__device__ __forceinline__ Limits limits(const GcGrid& g, int3 c, float rc) {
+    Limits l;
+    l.cross = 0;
+    auto axis = [&](int a, int cc, float& centre, float& own, float& cand) {
+        const float w = 1.f / g.invw[a];
+        centre = g.origin[a] + ((float)cc + 0.5f) * w;
+        own = cand = kFar;
+        if (!(g.pmask & (1 << a))) return;
+        if (cc == 0 || cc == g.n[a] - 1) {
+            l.cross |= 1 << a;
+            return;
+        }
+        const float spare = 0.5f * (g.L[a] * 0.99999f - rc) - w;
+        own = 0.5f * w + spare;
+        cand = 1.5f * w + spare;
+    };
+    axis(0, c.x, l.centre.x, l.own.x, l.cand.x);
+    axis(1, c.y, l.centre.y, l.own.y, l.cand.y);
+    axis(2, c.z, l.centre.z, l.own.z, l.cand.z);
+    return l;
+}
+
+// The form that a position asks for beyond l.cross.
+__device__ __forceinline__ int form_of(float3 x, const Limits& l, float3 lim) {
+    const float3 d = f3(fabsf(x.x - l.centre.x), fabsf(x.y - l.centre.y), fabsf(x.z - l.centre.z));
+    if (d.x <= lim.x && d.y <= lim.y && d.z <= lim.z) return 0;
+    return d.x < kFar && d.y < kFar && d.z < kFar ? 7 : kAny;
 }
 
 template <bool IMAGE>
@@ -114,18 +145,26 @@ __device__ __forceinline__ float3 diff(float3 a, float4 b, const GcGrid& g) {
 }
 
 // Marks the staged candidates [0, m) (m a multiple of 4 kGroup, padded with
-// far ones) within cut2 of xa and of xb that lane s tests; returns their
+// far ones) within cutm of xa and of xb that lane s tests; returns their
 // numbers (xa's in the low half).  Bit 31 - u of word w is the candidate
 // w * kWord + u * kGroup + s.
 //
-// The plain form takes seven instructions a candidate and particle: r^2 -
-// cut2 by fused multiply-adds and its sign shifted into the word (a pair
-// within a rounding of the cut-off, where every pair function here is zero,
-// may count or not).  With IMAGE the squared distance of the minimum image is
-// tested as the oracle tests it; a NaN distance counts as within, so that a
-// lost particle shows in its neighbours.
-template <bool IMAGE>
-__device__ __forceinline__ int mark(Shared& sh, float3 xa, float3 xb, int s, int m, float cut2, const GcGrid& g) {
+// The test takes seven instructions a candidate and particle, two more for an
+// axis with the image: r^2 - cutm by fused multiply-adds, where the image's
+// distance is the smaller of |d| and L - |d|, and its sign shifted into the
+// word.  cutm is the cut-off with a margin above its rounding; evaluate()
+// applies the predicate itself.
+template <int FORM>
+__device__ __forceinline__ int mark(Shared& sh, float3 xa, float3 xb, int s, int m, float cutm, const GcGrid& g) {
+    const float3 L = f3(g.pmask & 1 ? g.L[0] : INFINITY, g.pmask & 2 ? g.L[1] : INFINITY,
+                        g.pmask & 4 ? g.L[2] : INFINITY);
+    auto beyond = [&](float3 x, float4 y) {
+        float dx = __fsub_rn(x.x, y.x), dy = __fsub_rn(x.y, y.y), dz = __fsub_rn(x.z, y.z);
+        if constexpr (FORM & 1) dx = fminf(fabsf(dx), L.x - fabsf(dx));
+        if constexpr (FORM & 2) dy = fminf(fabsf(dy), L.y - fabsf(dy));
+        if constexpr (FORM & 4) dz = fminf(fabsf(dz), L.z - fabsf(dz));
+        return fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, -cutm)));
+    };
     int count = 0;
     for (int w = 0, q0 = 0; q0 < m; ++w, q0 += kWord) {
         const int it = min(32, (m - q0) / kGroup);
@@ -135,15 +174,13 @@ __device__ __forceinline__ int mark(Shared& sh, float3 xa, float3 xb, int s, int
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const float4 xj = x[(u0 + u) * kGroup];
-                const float3 da = diff<IMAGE>(xa, xj, g), db = diff<IMAGE>(xb, xj, g);
-                if constexpr (IMAGE) {
-                    a = (a << 1) | (norm2_rn(da) >= cut2 ? 0u : 1u);
-                    b = (b << 1) | (norm2_rn(db) >= cut2 ? 0u : 1u);
+                if constexpr (FORM == kAny) {
+                    const bool none = xj.x == kFar;
+                    a = (a << 1) | (none || norm2_rn(diff<true>(xa, xj, g)) >= cutm ? 0u : 1u);
+                    b = (b << 1) | (none || norm2_rn(diff<true>(xb, xj, g)) >= cutm ? 0u : 1u);
                 } else {
-                    const float ta = fmaf(da.x, da.x, fmaf(da.y, da.y, fmaf(da.z, da.z, -cut2)));
-                    const float tb = fmaf(db.x, db.x, fmaf(db.y, db.y, fmaf(db.z, db.z, -cut2)));
-                    a = __funnelshift_l(__float_as_uint(ta), a, 1);
-                    b = __funnelshift_l(__float_as_uint(tb), b, 1);
+                    a = __funnelshift_l(__float_as_uint(beyond(xa, xj)), a, 1);
+                    b = __funnelshift_l(__float_as_uint(beyond(xb, xj)), b, 1);
                 }
             }
         }
@@ -160,12 +197,13 @@ __device__ __forceinline__ int mark(Shared& sh, float3 xa, float3 xb, int s, int
 // this thread's particle (particle h of the group): lane s of its four takes
 // the ranks total s / 4 to total (s + 1) / 4 of the marks in the order of
 // lanes, words and bits.  (The marks found by four lanes differ by a third,
-// and the largest of a warp's shares sets its time.)  `count` as mark()
-// returned it.  Called by whole warps.
+// and the largest of a warp's shares sets its time.)  The marked candidates
+// within cut2 by the oracle's predicate, bit for bit, are the pairs.  `count`
+// as mark() returned it.  Called by whole warps.
 template <bool IMAGE, class Op>
 __device__ __forceinline__ void evaluate(const Op& op, const typename Op::Extra& ex, const typename Op::Self& self,
                                          typename Op::Acc& acc, const Shared& sh, float3 xi, int m, int count,
-                                         const GcParams& p) {
+                                         float cut2, const GcParams& p) {
     const int t = threadIdx.x % kGroup, h = t / kLanes, s = t % kLanes;
     int end = count;   // inclusive scan over the group's lanes
 #pragma unroll
@@ -209,22 +247,19 @@ __device__ __forceinline__ void evaluate(const Op& op, const typename Op::Extra&
         const int q = w * kWord + u * kGroup + lane;
         const float4 xj = sh.x[q];
         const float3 d = diff<IMAGE>(xi, xj, p.g);
-        op.pair(acc, self, ex, q, __float_as_uint(xj.w), d, IMAGE ? norm2_rn(d) : norm2_fma(d), p);
+        const float r2 = norm2_rn(d);
+        if (!(r2 >= cut2)) op.pair(acc, self, ex, q, __float_as_uint(xj.w), d, r2, p);
     }
 }
 
 // The sweep.  Op says which particles it is for (active), which candidates
 // take part (keep), what else of a candidate is staged (Extra, stage), the
 // cut-off, the pair function, what to do with the sum (finish) and with a
-// particle that it is not for (idle); with Op::kExact the neighbour predicate
-// is the oracle's, bit for bit.
+// particle that it is not for (idle).
 //
-// Positions are staged with the shift of their cube, and with every staged
-// position inside the box the plain difference of shifted positions is the
-// minimum image of every pair within a cube width (other pairs are beyond
-// the cut-off either way).  Where a staged position lies outside the box
-// (a caller that has not wrapped it), the unshifted positions are staged and
-// the image is formed pair by pair.
+// Positions are staged as they are; whether a cube's pairs need the minimum
+// image follows from its place in the grid and from the positions (Limits),
+// one form per cube.
 template <class Op>
 __global__ void __launch_bounds__(kBlock, Op::kBlocks) k_sweep(int K, int per_block, GcParams p, Op op,
                                                   const float3* __restrict__ coor, const int* __restrict__ sortpart,
@@ -233,39 +268,42 @@ __global__ void __launch_bounds__(kBlock, Op::kBlocks) k_sweep(int K, int per_bl
     __shared__ typename Op::Extra ex;
     const GcGrid& g = p.g;
     const int grp = threadIdx.x / kGroup, t = threadIdx.x % kGroup, h = t / kLanes;
+    const float cut2 = op.cut2(p), cutm = cut2 * 1.00001f;
     const int k1 = min(K, (int)(blockIdx.x + 1) * per_block);
     for (int cube = blockIdx.x * per_block; cube < k1; ++cube) {
         const int2 be = bec[cube];
         if (be.y <= be.x) continue;
-        bool any = false, own_out = false;
+        const int3 c = make_int3(cube % g.n[0], cube / g.n[0] % g.n[1], cube / g.n[0] / g.n[1]);
+        const Limits lim = limits(g, c, p.rc);
+        bool any = false;
+        int own_form = 0;
         for (int i = be.x + threadIdx.x; i < be.y; i += kBlock) {
             const unsigned id = (unsigned)sortpart[i];
             if (op.active(id, p)) {
                 any = true;
-                own_out |= outside(coor[i], g);
+                own_form |= form_of(coor[i], lim, lim.own);
             } else {
                 op.idle(i);
             }
         }
         if (!__syncthreads_or(any)) continue;
-        stencil(g, make_int3(cube % g.n[0], cube / g.n[0] % g.n[1], cube / g.n[0] / g.n[1]), bec, sh);
+        stencil(g, c, bec, sh);
         const int total = sh.off[27];
-        bool image = Op::kExact, some = false;
+        int form = 0;
+        bool some = false;
         // stages the candidates [q0, q0 + cnt), padded with far ones to m
-        auto stage = [&](int q0, int cnt, int m, bool shifted, bool& out) {
+        auto stage = [&](int q0, int cnt, int m, int& need) {
             bool kept = false;
             for (int r = threadIdx.x / 32; r < 27; r += kBlock / 32) {
                 const int o = sh.off[r] - q0, e = min(sh.off[r + 1] - q0, cnt), j0 = sh.beg[r] - o;
-                const float3 v = sh.shift[r];
                 for (int q = max(o, 0) + (int)threadIdx.x % 32; q < e; q += 32) {
                     const int j = j0 + q;
                     const unsigned idj = (unsigned)sortpart[j];
                     float4 x = make_float4(kFar, kFar, kFar, 0.f);
                     if (op.keep(idj, p)) {
                         const float3 y = coor[j];
-                        out |= outside(y, g);
-                        x = shifted ? make_float4(y.x + v.x, y.y + v.y, y.z + v.z, __uint_as_float(idj))
-                                    : make_float4(y.x, y.y, y.z, __uint_as_float(idj));
+                        need |= form_of(y, lim, lim.cand);
+                        x = make_float4(y.x, y.y, y.z, __uint_as_float(idj));
                         kept = true;
                         op.stage(ex, q, j, p);
                     }
@@ -280,7 +318,7 @@ __global__ void __launch_bounds__(kBlock, Op::kBlocks) k_sweep(int K, int per_bl
             const int ia = b0 + 2 * grp, i = ia + h;
             const unsigned id = i < be.y ? (unsigned)sortpart[i] : 0u;
             const bool act = i < be.y && op.active(id, p);
-            const float3 own = act ? coor[i] : f3(-kFar, -kFar, -kFar);
+            const float3 xi = act ? coor[i] : f3(-kFar, -kFar, -kFar);
             typename Op::Acc acc;
             typename Op::Self self;
             op.begin(acc, self, i, id, act, p);
@@ -289,30 +327,28 @@ __global__ void __launch_bounds__(kBlock, Op::kBlocks) k_sweep(int K, int per_bl
                 const int m = (cnt + 4 * kGroup - 1) / (4 * kGroup) * (4 * kGroup);
                 if (b0 == be.x || total > kCap) {   // the candidates stay staged for the cube's next particles
                     __syncthreads();
-                    bool out = own_out;
-                    const bool kept = stage(q0, cnt, m, !Op::kExact, out);
+                    int need = own_form;
+                    const bool kept = stage(q0, cnt, m, need);
                     some = __syncthreads_or(kept);
-                    if (!Op::kExact) {
-                        image = __syncthreads_or(out);
-                        if (image) {
-                            stage(q0, cnt, m, false, out);
-                            __syncthreads();
-                        }
-                    }
+                    form = lim.cross;
+                    if (__syncthreads_or(need)) form = __syncthreads_or(need & kAny) ? kAny : 7;
                 }
                 if (!some || !__any_sync(0xffffffffu, act)) continue;
-                auto both = [&](auto im) {
-                    constexpr bool I = decltype(im)::value;
-                    const float3 v = I ? f3(0.f, 0.f, 0.f) : sh.shift[13];
-                    const float3 xi = f3(own.x + v.x, own.y + v.y, own.z + v.z);
-                    const float3 xo = f3(__shfl_xor_sync(0xffffffffu, xi.x, kLanes), __shfl_xor_sync(0xffffffffu, xi.y, kLanes),
-                                         __shfl_xor_sync(0xffffffffu, xi.z, kLanes));
-                    const int count = mark<I>(sh, h ? xo : xi, h ? xi : xo, t, m, op.cut2(p), g);
-                    __syncwarp();
-                    evaluate<I>(op, ex, self, acc, sh, xi, m, count, p);
-                };
-                if (image) both(std::true_type{});
-                else both(std::false_type{});
+                const float3 xo = f3(__shfl_xor_sync(0xffffffffu, xi.x, kLanes), __shfl_xor_sync(0xffffffffu, xi.y, kLanes),
+                                     __shfl_xor_sync(0xffffffffu, xi.z, kLanes));
+                const float3 xa = h ? xo : xi, xb = h ? xi : xo;
+                int count;
+                switch (form) {
+                case 0: count = mark<0>(sh, xa, xb, t, m, cutm, g); break;
+                case 1: count = mark<1>(sh, xa, xb, t, m, cutm, g); break;
+                case 2: count = mark<2>(sh, xa, xb, t, m, cutm, g); break;
+                case 4: count = mark<4>(sh, xa, xb, t, m, cutm, g); break;
+                case kAny: count = mark<kAny>(sh, xa, xb, t, m, cutm, g); break;
+                default: count = mark<7>(sh, xa, xb, t, m, cutm, g);
+                }
+                __syncwarp();
+                if (form == 0) evaluate<false>(op, ex, self, acc, sh, xi, m, count, cut2, p);
+                else evaluate<true>(op, ex, self, acc, sh, xi, m, count, cut2, p);
                 __syncwarp();   // the marks are written again for the next candidates
             }
             op.reduce(acc);

@@ -30,10 +30,6 @@
 
 namespace {
 
-// Smallest normal number: squared distances below it (particles within 1e-19
-// of each other) count as zero, and rsqrt_ftz takes normal arguments only.
-constexpr float kTiny = 1.17549435e-38f;
-
 // K2 -- r += dt v + dt^2/2 F/m for fluid and membrane particles.
 __global__ void k_update_coor(int n, GcParams p, const int* __restrict__ sortpart, const float3* __restrict__ force,
                               float3* __restrict__ coor, const float4* __restrict__ velrhop, unsigned* flags) {
@@ -93,7 +89,7 @@ struct DensityOp {
     }
     __device__ void stage(Extra&, int, int, const GcParams&) const {}
     __device__ void pair(Acc& a, const Self& s, const Extra&, int, unsigned idj, float3, float r2, const GcParams& p) const {
-        if (idj != s.id) a.sum += wendland_w(r2 < kTiny ? 0.f : r2 * rsqrt_ftz(r2), p);
+        if (idj != s.id) a.sum += wendland_w(sqrtf(r2), p);
     }
     __device__ void reduce(Acc& a) const { a.sum = gcsweep::lane_sum(a.sum); }
     __device__ void finish(const Acc& a, const Self&, int i, const GcParams& p) const {
@@ -138,7 +134,7 @@ struct Bound2VelOp {
         e.v[q] = f3(v.x, v.y, v.z);
     }
     __device__ void pair(Acc& a, const Self&, const Extra& e, int q, unsigned, float3, float r2, const GcParams& p) const {
-        const float w = wendland_w(r2 < kTiny ? 0.f : r2 * rsqrt_ftz(r2), p);
+        const float w = wendland_w(sqrtf(r2), p);
         a.num += w * e.v[q];
         a.den += w;
     }
@@ -175,10 +171,14 @@ __global__ void k_eos(int n, GcParams p, const int* __restrict__ sortpart, const
 }
 
 // K12 -- SDPD pair force; writes the force of every slot (zero for walls).
-// A candidate's velocity, 1/d and P/d^2 are staged with its position.  The
+// A candidate's velocity, d and P/d^2 are staged with its position.  The
 // pair terms are gathered into one coefficient along d = x_i - x_j (pressure
-// and the e e^T parts of the viscous and random forces, e = d/r folded in as
-// 1/r^2), one along v_ij and one along xi_ij, as in the fused step.
+// and the e e^T parts of the viscous and random forces, e = d/r), one along
+// v_ij and one along xi_ij, as in the fused step.  Roots and divisions are the
+// correctly rounded ones, here and in the other sweeps: with rsqrt.approx and
+// a product of two reciprocals a million-particle step took 3.06 instead of
+// 3.24 ms, but a pair near the cut-off, where F goes as (1 - r/rc)^3, was off
+// by twice as much.
 template <bool NOISE>
 struct SdpdOp {
     const float4* velrhop;
@@ -186,7 +186,7 @@ struct SdpdOp {
     float3* force;
     static constexpr int kBlocks = 6;   // resident blocks the registers are cut to
     struct Extra { float4 v[gcsweep::kCap]; float pt[gcsweep::kCap]; };
-    struct Self { float3 v; float inv_d, pt; unsigned id; };
+    struct Self { float3 v; float d, pt; unsigned id; };
     struct Acc { float3 f; };
     __device__ float cut2(const GcParams& p) const { return p.rc2; }
     __device__ bool active(unsigned id, const GcParams& p) const { return is_mobile(id, p); }
@@ -198,33 +198,32 @@ struct SdpdOp {
         const float4 v = velrhop[i];
         const float d = v.w * p.inv_mass;
         s.v = f3(v.x, v.y, v.z);
-        s.inv_d = 1.f / d;
+        s.d = d;
         s.pt = press[i] / (d * d);
         s.id = id;
     }
     __device__ void stage(Extra& e, int q, int j, const GcParams& p) const {
         const float4 v = velrhop[j];
         const float d = v.w * p.inv_mass;
-        e.v[q] = make_float4(v.x, v.y, v.z, 1.f / d);
+        e.v[q] = make_float4(v.x, v.y, v.z, d);
         e.pt[q] = press[j] / (d * d);
     }
     __device__ void pair(Acc& a, const Self& s, const Extra& e, int q, unsigned idj, float3 d, float r2,
                          const GcParams& p) const {
-        if (r2 < kTiny || idj == s.id) return;   // coincident particles exert no force
+        if (r2 <= 0.f || idj == s.id) return;   // coincident particles exert no force
         const float4 vj = e.v[q];
-        const float inv_r = rsqrt_ftz(r2), ir2 = inv_r * inv_r;
-        const float F = wendland_f(r2 * inv_r, p);
+        const float r = sqrtf(r2), inv_r = 1.f / r;
+        const float F = wendland_f(r, p);
         const float3 vij = f3(s.v.x - vj.x, s.v.y - vj.y, s.v.z - vj.z);
-        const float fdd = F * (s.inv_d * vj.w);
-        float cd = (s.pt + e.pt[q]) * F - (fdd * p.visB) * dot3(d, vij) * ir2;
+        const float fdd = F / (s.d * vj.w);
+        float cd = (s.pt + e.pt[q]) * F - (fdd * p.visB) * (dot3(d, vij) * inv_r) * inv_r;
         a.f += (-fdd * p.visA) * vij;
         if constexpr (NOISE) {
             // a pair at the cut-off can give F a rounding-sized negative value: no noise then
-            const float qq = p.noise_pref * fdd;
-            float n = qq >= kTiny ? qq * rsqrt_ftz(qq) : 0.f;
+            float n = fdd > 0.f ? sqrtf(p.noise_pref * fdd) : 0.f;
             n = s.id < idj ? n : -n;   // the pair sign of xi_ij
             const float3 xi = pair_noise_unsigned(s.id, idj, p);
-            cd += (n * (p.sqrtAB - p.sqrtA)) * dot3(d, xi) * ir2;
+            cd += (n * (p.sqrtAB - p.sqrtA)) * (dot3(d, xi) * inv_r) * inv_r;
             a.f += (n * p.sqrtA) * xi;
         }
         a.f += cd * d;

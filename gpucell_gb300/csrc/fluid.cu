@@ -264,7 +264,7 @@ template <class Op>
 int launch_sweep(const Op& op, int n, const GcParams& p, const float* coor, const int* sortpart, const int* bec,
                  cudaStream_t st, const char* what) {
     const int K = p.g.ncells, per = gcsweep::cubes_per_block(n, K);
-    gcsweep::k_sweep<<<gc_blocks(K, per), gcsweep::kBlock, 0, st>>>(K, per, p, op, (const float3*)coor, sortpart,
+    gcsweep::k_sweep<<<gc_blocks(K, per), gcsweep::kBlock, 0, st>>>(K, p, op, (const float3*)coor, sortpart,
                                                                     (const int2*)bec);
     GC_CHECK_LAUNCH(what);
     return GC_OK;

@@ -330,7 +330,7 @@ constexpr int kAggPart = kAggBlock / kAggLanes;    // vertices of a cube taken t
 constexpr int kAggCap = 352;                       // kept candidates per warp
 constexpr int kAggAhead = 4;                       // ids in flight per lane
 
-__global__ void __launch_bounds__(kAggBlock, 4) k_aggregate(int K, int per_block, GcParams p, int R0, int R1, int R2,
+__global__ void __launch_bounds__(kAggBlock, 4) k_aggregate(int K, GcParams p, int R0, int R1, int R2,
                                                             const float3* __restrict__ coor,
                                                             const int* __restrict__ sortpart,
                                                             const int* __restrict__ celltab,
@@ -341,10 +341,13 @@ __global__ void __launch_bounds__(kAggBlock, 4) k_aggregate(int K, int per_block
     __shared__ int own[kAggPart], scnt[kAggWarps], sdone[kAggWarps], snext;
     const GcGrid& g = p.g;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, s = threadIdx.x % kAggLanes;
-    const int k1 = min(K, (int)(blockIdx.x + 1) * per_block);
     const int ny = 2 * R1 + 1, rows = 2 * ny * (2 * R2 + 1);   // two ranges per row of the stencil
-    for (int cube = blockIdx.x * per_block; cube < k1; ++cube) {
+    for (int cube = blockIdx.x; cube < K; cube += gridDim.x) {   // as in k_sweep
         const int2 be = bec[cube];
+        if (be.y <= be.x) {
+            cube = gcsweep::last_empty(cube, K, bec);
+            continue;
+        }
         bool any = false;
         for (int i = be.x + threadIdx.x; i < be.y; i += kAggBlock) any |= (unsigned)sortpart[i] >= p.nC;
         if (!__syncthreads_or(any)) continue;
@@ -616,7 +619,7 @@ int gc_cupar_CalCellAggForce(unsigned ncell, unsigned n, unsigned ncellpar, floa
     }
     const int K = p.g.ncells, per = gcsweep::cubes_per_block(n, K);
     k_aggregate<<<gc_blocks(K, per), kAggBlock, 0, s.stream>>>(
-        K, per, p, R[0], R[1], R[2], (const float3*)d_totalcoor, d_sortpart, d_celltab, (const int2*)d_beginendcube,
+        K, p, R[0], R[1], R[2], (const float3*)d_totalcoor, d_sortpart, d_celltab, (const int2*)d_beginendcube,
         d_pararea, (float3*)d_aggforce, (float3*)d_totalforce);
     GC_CHECK_LAUNCH("CalCellAggForce");
     return GC_OK;

@@ -51,6 +51,22 @@ inline int cubes_per_block(long long n, long long K) {
     return c < 1 ? 1 : (c > 128 ? 128 : (int)c);
 }
 
+// A block takes every gridDim-th cube, so that a crowd of particles in a
+// corner of a sparse grid is shared out over the blocks.  From an empty cube
+// on, the block's next 32 are looked at together, as the empty cubes of such a
+// grid would otherwise be a serial chain of loads: last_empty gives the last
+// of the empty ones.  Density of 10 / 80 / 27 thousand particles crowded into 0.04
+// / 0.3 / 0.8 % of a box: 301 / 315 / 200 us with runs of consecutive cubes per
+// block, 199 / 322 / 69 with every gridDim-th cube, 48 / 172 / 58 with both.
+// Called by whole warps.
+__device__ __forceinline__ int last_empty(int cube, int K, const int2* __restrict__ bec) {
+    const long long step = gridDim.x, c = cube + ((threadIdx.x & 31) + 1) * step;
+    const int2 be = c < K ? bec[c] : make_int2(0, 0);
+    const unsigned full = __ballot_sync(0xffffffffu, be.y > be.x);
+    const long long last = cube + (full ? __ffs(full) - 1 : 32) * step;
+    return last < K ? (int)last : K;
+}
+
 struct Shared {
     float4 x[kCap];                      // position, id bits
     unsigned mark[2][kWords * kBlock];   // per particle of the group: word w of thread t at w * kBlock + t
@@ -261,7 +277,7 @@ __device__ __forceinline__ void evaluate(const Op& op, const typename Op::Extra&
 // image follows from its place in the grid and from the positions (Limits),
 // one form per cube.
 template <class Op>
-__global__ void __launch_bounds__(kBlock, Op::kBlocks) k_sweep(int K, int per_block, GcParams p, Op op,
+__global__ void __launch_bounds__(kBlock, Op::kBlocks) k_sweep(int K, GcParams p, Op op,
                                                   const float3* __restrict__ coor, const int* __restrict__ sortpart,
                                                   const int2* __restrict__ bec) {
     __shared__ Shared sh;
@@ -269,10 +285,12 @@ __global__ void __launch_bounds__(kBlock, Op::kBlocks) k_sweep(int K, int per_bl
     const GcGrid& g = p.g;
     const int grp = threadIdx.x / kGroup, t = threadIdx.x % kGroup, h = t / kLanes;
     const float cut2 = op.cut2(p), cutm = cut2 * 1.00001f;
-    const int k1 = min(K, (int)(blockIdx.x + 1) * per_block);
-    for (int cube = blockIdx.x * per_block; cube < k1; ++cube) {
+    for (int cube = blockIdx.x; cube < K; cube += gridDim.x) {
         const int2 be = bec[cube];
-        if (be.y <= be.x) continue;
+        if (be.y <= be.x) {
+            cube = last_empty(cube, K, bec);
+            continue;
+        }
         const int3 c = make_int3(cube % g.n[0], cube / g.n[0] % g.n[1], cube / g.n[0] / g.n[1]);
         const Limits lim = limits(g, c, p.rc);
         bool any = false;

@@ -202,13 +202,40 @@ __global__ void fk_integrate(int n, GcParams p, SysInfo s0, const SysInfo* __res
 // ---------------------------------------------------------------------------
 // Rebuild: cube keys, permutation, neighbour lists
 // ---------------------------------------------------------------------------
+// Wraps the double-float position (x, l) into [lo, hi] of a periodic axis and
+// returns the crossings.  The FP32 part can come out as hi itself (a particle
+// less than half an ulp below lo).
+__device__ __forceinline__ int wrap_axis(float& x, float& l, const GcGrid& g, int a, int ddpos) {
+    if (!(g.pmask & (1 << a)) || !isfinite(x)) return 0;
+    int w = (int)floorf((x - g.lo[a]) / g.L[a]);
+    if (w != 0) {
+        pos_add(x, l, -(float)w * g.L[a], ddpos);
+        if (x >= g.hi[a]) { pos_add(x, l, -g.L[a], ddpos); ++w; }
+        else if (x < g.lo[a]) { pos_add(x, l, g.L[a], ddpos); --w; }
+    }
+    return w;
+}
+
+// List-grid cell of a wrapped coordinate.  At a periodic face it stays on the
+// side that the coordinate is on (hi, and floats below it whose product rounds
+// up to the number of cells, are of the last cell), as the list build takes
+// the image shift of a pair of cells from their indices.
+__device__ __forceinline__ int list_coord(float x, int axis, const GcGrid& g) {
+    const int c = (int)floorf(__fmul_rn(__fsub_rn(x, g.origin[axis]), g.invw[axis]));
+    return min(max(c, 0), g.n[axis] - 1);
+}
+
 __global__ void fk_cellkey(int n, const SysInfo* __restrict__ sys, const int* __restrict__ sysid,
-                           const float4* __restrict__ pos, int* __restrict__ keys, int* __restrict__ vals) {
+                           const float4* __restrict__ pos, const float4* __restrict__ plo, int* __restrict__ keys,
+                           int* __restrict__ vals, int ddpos) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const SysInfo& S = sys[sysid ? sysid[i] : 0];
-    float4 x = pos[i];
-    keys[i] = S.cube0 + cube_key(cube_coord(x.x, 0, S.g), cube_coord(x.y, 1, S.g), cube_coord(x.z, 2, S.g), S.g);
+    float4 x = pos[i], lo = plo[i];
+    wrap_axis(x.x, lo.x, S.g, 0, ddpos);   // as fk_permute will
+    wrap_axis(x.y, lo.y, S.g, 1, ddpos);
+    wrap_axis(x.z, lo.z, S.g, 2, ddpos);
+    keys[i] = S.cube0 + cube_key(list_coord(x.x, 0, S.g), list_coord(x.y, 1, S.g), list_coord(x.z, 2, S.g), S.g);
     vals[i] = i;
 }
 
@@ -225,22 +252,9 @@ __global__ void fk_permute(int n, const SysInfo* __restrict__ sys, const int* __
     const GcGrid& g = sys[s].g;
     float4 x = src.pos[o], lo = src.plo[o];
     int4 t = src.nthro[o];
-    float* xs[3] = {&x.x, &x.y, &x.z};
-    float* ls[3] = {&lo.x, &lo.y, &lo.z};
-    int* ts[3] = {&t.x, &t.y, &t.z};
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if (!(g.pmask & (1 << a))) continue;
-        float c = *xs[a];
-        if (!isfinite(c)) continue;
-        int w = (int)floorf((c - g.lo[a]) / g.L[a]);
-        if (w != 0) {
-            pos_add(*xs[a], *ls[a], -(float)w * g.L[a], ddpos);
-            if (*xs[a] >= g.hi[a]) { pos_add(*xs[a], *ls[a], -g.L[a], ddpos); ++w; }
-            else if (*xs[a] < g.lo[a]) { pos_add(*xs[a], *ls[a], g.L[a], ddpos); --w; }
-            *ts[a] += w;
-        }
-    }
+    t.x += wrap_axis(x.x, lo.x, g, 0, ddpos);
+    t.y += wrap_axis(x.y, lo.y, g, 1, ddpos);
+    t.z += wrap_axis(x.z, lo.z, g, 2, ddpos);
     dst.pos[q] = x;
     dst.plo[q] = lo;
     dst.vel[q] = src.vel[o];
@@ -336,7 +350,7 @@ __device__ __forceinline__ int scan_rows(int r0, int r1, int k, int i, float3 xi
     const unsigned fl = S.fl;
     const bool mobile_only = t == PT_B2;
     const int R = S.lr, side = 2 * R + 1;
-    const int cx = cube_coord(xi.x, 0, g), cy = cube_coord(xi.y, 1, g), cz = cube_coord(xi.z, 2, g);
+    const int cx = list_coord(xi.x, 0, g), cy = list_coord(xi.y, 1, g), cz = list_coord(xi.z, 2, g);
     const float cut = sqrtf(cut2), eps = 2e-3f;
     const float lim2 = (cut + eps) * (cut + eps);
     for (int r = r0; r < r1; ++r) {
@@ -370,8 +384,8 @@ __device__ __forceinline__ int scan_rows(int r0, int r1, int k, int i, float3 xi
             else if (x >= g.n[0]) { if (!(g.pmask & 1)) continue; x -= g.n[0]; sx = -g.L[0]; }
             const unsigned jb = start[row + x], je = start[row + (whole ? b : x) + 1];
             const float3 xs = f3(xi.x + sx, xi.y + sy, xi.z + sz);
-            // (slot i may lie in another row than its own: it was sorted by the
-            // position before the wrap, which rounds)
+            // (the row with slot i itself: its own, or another one after the
+            // restore of a checkpoint whose cells were those before the wrap)
             if (mobile_only || (unsigned)i - jb < je - jb || k + (int)(je - jb) > cap)
                 scan_range<WRITE, true>(pos, jb, je, xs, i, cut2, mobile_only, fl, cap, lst, k);
             else
@@ -1979,7 +1993,7 @@ int rebuild_lists(GcFused* f) {
     const int n = f->n;
     const int nb = gc_blocks(n, f->block);
     cudaStream_t st = f->st;
-    fk_cellkey<<<nb, f->block, 0, st>>>(n, f->dsys, f->a.sys, f->a.pos, f->keys, f->vals);
+    fk_cellkey<<<nb, f->block, 0, st>>>(n, f->dsys, f->a.sys, f->a.pos, f->a.plo, f->keys, f->vals, f->ddpos);
     GC_CHECK_LAUNCH("fused: cube keys");
     GC_TRY(gc_counting_sort_bufs(n, f->K, f->keys, f->vals, f->sb, f->flags, st));
     fk_permute<<<nb, f->block, 0, st>>>(n, f->dsys, f->vals, f->a, f->b, f->refpos, f->slot_of, f->ddpos);
@@ -2285,7 +2299,7 @@ int one_step(GcFused* f, int drive) {
 // the call's steps and recovers from).
 int launch_rebuild_body(GcFused* f, cudaStream_t st) {
     const int n = f->n, nb = gc_blocks(n, f->block);
-    fk_cellkey<<<nb, f->block, 0, st>>>(n, f->dsys, f->a.sys, f->a.pos, f->keys, f->vals);
+    fk_cellkey<<<nb, f->block, 0, st>>>(n, f->dsys, f->a.sys, f->a.pos, f->a.plo, f->keys, f->vals, f->ddpos);
     GC_CHECK_LAUNCH("fused: cube keys");
     GC_TRY(gc_counting_sort_bufs(n, f->K, f->keys, f->vals, f->sb, f->flags, st));
     fk_permute<<<nb, f->block, 0, st>>>(n, f->dsys, f->vals, f->a, f->b, f->refpos, f->slot_of, f->ddpos);

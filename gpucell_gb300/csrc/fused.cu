@@ -1357,7 +1357,7 @@ __global__ void fk_mgather(int ncp, int nedge, const int* __restrict__ inc_ptr, 
     parea[v] = a;
 }
 
-// Morse aggregation on membrane-only grids (cubes at least MaxCut wide).
+// Morse aggregation on membrane-only grids (agg_grid).
 __global__ void fk_mkey(int ncp, const SysInfo* __restrict__ sys, const int* __restrict__ msys,
                         const float4* __restrict__ mpos, int* __restrict__ keys, int* __restrict__ vals) {
     int v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1421,8 +1421,7 @@ __device__ __forceinline__ void morse_run(const GcParams& p, const GcGrid& g, fl
 // only the listed pairs.
 //
 // The list build (fk_mlist) runs a warp per vertex over the (2R+1)^3
-// aggregation cubes around it (R = 2 for cubes at least MaxCut/2 wide, 1 for
-// cubes at least MaxCut wide).  The lanes test 32 cubes at a time (cubes
+// aggregation cubes around it (agg_grid: the stencil reaches MaxCut + skin).  The lanes test 32 cubes at a time (cubes
 // farther than the cut-off are not read) and then go through each cube that
 // is left together, lane k taking the candidates k, k + 32, ...: consecutive
 // loads and no lane waiting for another.  A first pass counts, a scan places
@@ -1888,6 +1887,33 @@ int build_morse_lists_from_ref(GcFused* f, cudaStream_t st) {
     return build_morse_lists(f, st, f->mref, true);
 }
 
+// Aggregation grid of a box: cubes for lists that reach cutl (MaxCut + skin)
+// by a stencil of radius *R.  Half-width cubes cut the candidates by ~40 %;
+// without five of them along every periodic axis cubes of cutl.  The box has
+// to take three cubes of MaxCut, or five of half of it, along each periodic
+// axis; one that does but not three of cutl is cut in three all the same: the
+// stencil then covers it whole.
+int agg_grid(const float* bbox, float maxcut, float cutl, int mask, GcGrid* g, int* R) {
+    auto half_width = [&](float cut) {
+        return gc_build_grid(bbox, 0.5f * cut, mask, g) == GC_OK && (!(mask & 1) || g->n[0] >= 5) &&
+               (!(mask & 2) || g->n[1] >= 5) && (!(mask & 4) || g->n[2] >= 5);
+    };
+    if (!half_width(maxcut)) GC_TRY(gc_build_grid(bbox, maxcut, mask, g));
+    *R = 2;
+    if (half_width(cutl)) return GC_OK;
+    *R = 1;
+    g->ncells = 1;
+    for (int a = 0; a < 3; ++a) {
+        const bool per = (mask >> a) & 1;
+        const double span = per ? (double)g->L[a] : (double)g->L[a] + 2.0 * cutl;
+        g->n[a] = std::max((int)floor(span / ((double)cutl * (1.0 + 1e-4))), per ? 3 : 1);
+        g->origin[a] = per ? g->lo[a] : g->lo[a] - cutl;
+        g->invw[a] = (float)(g->n[a] / span);
+        g->ncells *= g->n[a];   // no more than with MaxCut
+    }
+    return GC_OK;
+}
+
 // Per-system list grids (cubes at least rc + skin wide) and aggregation
 // grids, their global cube offsets, and the device copy of the table.
 int build_grids(GcFused* f) {
@@ -1924,15 +1950,7 @@ int build_grids(GcFused* f) {
         S.cube0 = K;
         K += S.g.ncells;
         if (f->have_agg) {
-            // the same for the aggregation grid: half-width cubes cut the
-            // candidates of the Morse pass by ~40 %
-            S.mlr = 2;
-            if (gc_build_grid(d.bbox, 0.5f * f->p.maxcut, d.periodic_mask, &S.mg) != GC_OK ||
-                ((d.periodic_mask & 1) && S.mg.n[0] < 5) || ((d.periodic_mask & 2) && S.mg.n[1] < 5) ||
-                ((d.periodic_mask & 4) && S.mg.n[2] < 5)) {
-                S.mlr = 1;
-                GC_TRY(gc_build_grid(d.bbox, f->p.maxcut, d.periodic_mask, &S.mg));
-            }
+            GC_TRY(agg_grid(d.bbox, f->p.maxcut, f->p.maxcut + f->skin, d.periodic_mask, &S.mg, &S.mlr));
             S.mcube0 = Kagg;
             Kagg += S.mg.ncells;
         } else {

@@ -86,9 +86,9 @@ struct SysInfo {
     float gx;                        // body force in x (ConstExtForce)
     float invL[3];
     int lr;                          // list-grid stencil radius: 2 for cells >= (rc + skin)/2, 1 for cubes >= rc + skin
-    int mlr;                         // aggregation-grid stencil radius: 2 for cubes >= MaxCut/2, 1 for cubes >= MaxCut
+    int mlr;                         // aggregation-grid stencil radius (agg_grid)
     GcGrid g;                        // list grid over the box
-    GcGrid mg;                       // aggregation grid: cubes at least MaxCut wide
+    GcGrid mg;                       // aggregation grid: stencils reach MaxCut + skin
 };
 
 // Particle type, system lookup, box constants and the minimum image of a

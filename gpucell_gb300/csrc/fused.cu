@@ -98,9 +98,14 @@ __device__ __forceinline__ unsigned near_axes(float3 x, const GcGrid& g, float m
 // of sixteen systems of 8 to 60 thousand particles takes 287 us without EACH and
 // 279 with it, at 524 k 335 and 330; the density pass of a 488 k constriction
 // 149 and 141, but that of the ensemble 110 and 117 (more registers).
+// `axes` by warp_axes, before any of the warp's threads returns: the lanes of
+// a particle exchange values within `run`, so they have to be in the same form.
+__device__ __forceinline__ unsigned warp_axes(bool live, float3 x, const GcGrid& g, float margin) {
+    return __reduce_or_sync(0xffffffffu, live ? near_axes(x, g, margin) : 0u);
+}
+
 template <bool EACH, class Run>
 __device__ __forceinline__ void run_near(unsigned axes, Run&& run) {
-    axes = __reduce_or_sync(__activemask(), axes);
     if (axes == 0) return run(std::integral_constant<int, 0>{});
     if constexpr (EACH) {
         if (axes == 1) return run(std::integral_constant<int, 1>{});
@@ -595,8 +600,8 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
         return;
     }
     const int q = (blockIdx.x - wall_blocks) * blockDim.x + threadIdx.x;
-    const int i = q / L, s = q % L;
-    if (i >= n) return;
+    const bool in = q / L < n;
+    const int i = in ? q / L : n - 1, s = q % L;
     float4 xi4 = pos[i];
     float3 xi = xyz(xi4);
     unsigned id = fid(xi4);
@@ -604,8 +609,10 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
     const Box B = box_of(S);
     const unsigned b2 = S.b2;
     int t = stype(id, S);
-    if (t != PT_FLUID && t != PT_MEMB) {
-        if (s == 0) {
+    const bool live = in && (t == PT_FLUID || t == PT_MEMB);
+    const unsigned axes = warp_axes(live, xi, S.g, wrap_margin);
+    if (!live) {
+        if (in && s == 0) {
             dp[i] = make_float2(p.mass / p.rho0, 0.f);
             if (t == PT_B1) rec[i] = PairRec{xi4, make_float4(0.f, 0.f, 0.f, 0.f)};
         }
@@ -673,7 +680,7 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
             }
         }
     };
-    run_near<!ENS>(near_axes(xi, S.g, wrap_margin), run);
+    run_near<!ENS>(axes, run);
     acc = group_sum<L>(acc, gm);
     if (s != 0) return;
     if (ccnt) ccnt[i] = kc;
@@ -748,16 +755,18 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
     if (skip && *skip) return;
     constexpr int G = L > 1 ? 2 : kForceGroup;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = q / L, ln = q % L;
-    if (i >= n) return;
+    const bool in = q / L < n;
+    const int i = in ? q / L : n - 1, ln = q % L;
     const PairRec ri = load_rec(rec + i);
     const float4 xi4 = ri.x;
     float3 xi = xyz(xi4);
     unsigned id = fid(xi4);
     const int s = ENS ? (sysid ? sysid[i] : 0) : 0;
     GC_SYS_OF(S, i);
-    if (id < S.fl) {
-        if (ln == 0) force[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool live = in && id >= S.fl;
+    const unsigned axes = warp_axes(live, xi, S.g, wrap_margin);
+    if (!live) {
+        if (in && ln == 0) force[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
     const Box B = box_of(S);
@@ -922,7 +931,7 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
             }
         }
     };
-    run_near<true>(near_axes(xi, S.g, wrap_margin), run);
+    run_near<true>(axes, run);
     float3 f = f3(fxy.x, fxy.y, fz);
     if constexpr (L > 1) {
         const unsigned gm = group_mask<L>();

@@ -734,6 +734,13 @@ struct PhiloxKeys {
     uint32_t k[10];
 };
 
+// What a pair of the force pass needs of the neighbour.
+struct Partner {
+    float4 x;          // position, id bits
+    float4 v;          // predicted velocity
+    float inv_d, pt;   // 1/d, P/d^2
+};
+
 __device__ __forceinline__ PairRec load_rec(const PairRec* p) {
     PairRec r;
     asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -747,7 +754,8 @@ __device__ __forceinline__ PairRec load_rec(const PairRec* p) {
 template <bool COMPACT, bool ENS, bool HALFV, bool NOISE, bool B1, int L, bool KEYS>
 __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
     fk_force(int n, GcParams p, SysInfo s0, const SysInfo* __restrict__ sys, const int* __restrict__ sysid,
-             const unsigned* __restrict__ nkey, const PairRec* __restrict__ rec, const float4* __restrict__ vh,
+             const unsigned* __restrict__ nkey, const PairRec* __restrict__ rec, const float4* __restrict__ pos,
+             const float4* __restrict__ vpred, const float2* __restrict__ dp, const float4* __restrict__ vh,
              float4* __restrict__ force, float4* __restrict__ vel, const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
              const unsigned* __restrict__ cmask, int mw, const float4* __restrict__ mforce, int drive,
              const uint2* __restrict__ vph, float wrap_margin, PhiloxKeys pk,
@@ -788,8 +796,9 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
         const float c2 = B1 ? (pid >= S.cs ? p.c2sq : p.c1sq) : p.c1sq;
         return (c2 * inv_d) * fmaf(-p.rho0, z, p.rest_m);
     };
-    const float idi = p.rest_invd + vi.w;   // 1/d
-    const float pti = pterm(vi.w, idi, id);
+    constexpr bool apart = HALFV;   // gathers from the arrays instead of the records
+    const float idi = apart ? dp[i].x : p.rest_invd + vi.w;   // 1/d
+    const float pti = apart ? dp[i].y : pterm(vi.w, idi, id);
     float2 fxy = make_float2(0.f, 0.f);
     float fz = 0.f;
     const int call = cnt[i];
@@ -852,8 +861,8 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
         fxy = make_float2(fmaf(c, axy.x, fxy.x), fmaf(c, axy.y, fxy.y));
         fz = fmaf(c, az, fz);
     };
-    // one pair: the neighbour's record
-    auto pair = [&](auto wrapc, PairRec rj) {
+    // one pair: the neighbour's position and id, velocity, 1/d and P/d^2
+    auto pair = [&](auto wrapc, const Partner& rj) {
         const float3 d = pair_diff<decltype(wrapc)::value>(xi, xyz(rj.x), B);
         const float2 dxy = make_float2(d.x, d.y);
         const float dz = d.z;
@@ -871,10 +880,9 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
         const float F = wendland_f(r2 * inv_r, p);
         const float2 vxy = __ffma2_rn(make_float2(rj.v.x, rj.v.y), make_float2(-1.f, -1.f), make_float2(vi.x, vi.y));
         const float vz = vi.z - rj.v.z;
-        const float idd = p.rest_invd + rj.v.w;
-        const float fdd = F * (idi * idd);
+        const float fdd = F * (idi * rj.inv_d);
         const float dv = fmaf(dxy.x, vxy.x, fmaf(dxy.y, vxy.y, dz * vz));
-        float cd = (pti + pterm(rj.v.w, idd, idj)) * F - (fdd * p.visB) * dv * ir2;
+        float cd = (pti + rj.pt) * F - (fdd * p.visB) * dv * ir2;
         add_f(-fdd * p.visA, vxy, vz);
         if constexpr (NOISE) {
             // (a pair at the cut-off can give F a rounding-sized negative value: its noise is as small)
@@ -891,16 +899,18 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
         }
         add_f(cd, dxy, dz);
     };
-    auto gather = [&](int j) -> PairRec {
-        PairRec r = load_rec(rec + j);
-        if constexpr (HALFV) {
-            const float w = r.v.w;
-            r.v = unpack_vel(vph[j]);
-            r.v.w = w;
+    auto gather = [&](auto apartc, int j) -> Partner {
+        if constexpr (decltype(apartc)::value) {
+            const float4 x = pos[j];
+            const float2 q = dp[j];
+            return Partner{x, HALFV ? unpack_vel(vph[j]) : vpred[j], q.x, q.y};
+        } else {
+            const PairRec r = load_rec(rec + j);
+            const float inv_d = p.rest_invd + r.v.w;
+            return Partner{r.x, r.v, inv_d, pterm(r.v.w, inv_d, fid(r.x))};
         }
-        return r;
     };
-    auto run = [&](auto wrapc) {
+    auto run = [&](auto wrapc, auto apartc) {
         {
             int jq[A][G];
 #pragma unroll
@@ -911,9 +921,9 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
                     jq[a][u] = k < c ? __ldg(lp + (size_t)next_k(k) * 32) : i;
                 }
             for (int k0 = 0; k0 < c; k0 += G) {
-                PairRec rg[G];
+                Partner rg[G];
 #pragma unroll
-                for (int u = 0; u < G; ++u) rg[u] = gather(jq[0][u]);
+                for (int u = 0; u < G; ++u) rg[u] = gather(apartc, jq[0][u]);
 #pragma unroll
                 for (int a = 0; a + 1 < A; ++a)
 #pragma unroll
@@ -931,7 +941,7 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
             }
         }
     };
-    run_near<true>(axes, run);
+    run_near<true>(axes, [&](auto w) { run(w, std::bool_constant<apart>{}); });
     float3 f = f3(fxy.x, fxy.y, fz);
     if constexpr (L > 1) {
         const unsigned gm = group_mask<L>();
@@ -2159,7 +2169,7 @@ void force_launch_n(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
     for (int r = 0; r < 10; ++r) pk.k[r] = p.noise_key + 0x9E3779B9u * (unsigned)r;
     auto go = [&](auto ens, auto keys) {
         fk_force<COMPACT, decltype(ens)::value, HALFV, NOISE, B1, L, decltype(keys)::value><<<nb, f->block, 0, st>>>(
-            n, p, s0(f), f->dsys, f->a.sys, nk, f->rec, f->a.vh, f->a.force, f->a.vel, f->nbr, c, f->cap, cm,
+            n, p, s0(f), f->dsys, f->a.sys, nk, f->rec, f->a.pos, f->a.vpred, f->dp, f->a.vh, f->a.force, f->a.vel, f->nbr, c, f->cap, cm,
             f->mw, mf, drive, f->vph, wrap_margin(f), pk, f->skip);
     };
     if (f->ens) go(std::true_type{}, std::false_type{});

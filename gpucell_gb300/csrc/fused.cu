@@ -117,7 +117,8 @@ __device__ __forceinline__ void run_near(unsigned axes, Run&& run) {
 
 // ---------------------------------------------------------------------------
 // Step prologue on the device: advance the step counter, derive every
-// system's noise key for the new step, clear the rebuild flag.
+// system's noise key for the new step, clear the rebuild flag and the word
+// for particles far above the rest density.
 // ---------------------------------------------------------------------------
 __global__ void fk_step_begin(int nsys, const SysInfo* __restrict__ sys, long long* __restrict__ dstep,
                               unsigned* __restrict__ nkey, int* __restrict__ rebuild) {
@@ -126,7 +127,7 @@ __global__ void fk_step_begin(int nsys, const SysInfo* __restrict__ sys, long lo
     __syncthreads();
     if (threadIdx.x == 0) {
         *dstep = s;
-        *rebuild = 0;
+        rebuild[0] = rebuild[1] = 0;
     }
 }
 
@@ -578,6 +579,12 @@ __global__ void fk_wallvel(int nwall, int n, GcParams p, SysInfo s0, const SysIn
 #define GC_DENS_MIN_BLOCKS 5
 #endif
 
+// The pair record holds 1/d as its distance from 1/d0, whose sum has an error
+// of u (1/d0 + ...): far above the rest density that is more than 1/d's own.
+// Beyond kDense times the rest density the density pass raises a word, and the
+// force pass of the step gathers 1/d and P/d^2 as they were computed.
+constexpr float kDense = 2.f;
+
 // A pass with `skip` set does nothing where that word is non-zero: it was
 // queued before the host knew that the lists have to be rebuilt first.
 //
@@ -592,7 +599,8 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
                                                   const int* __restrict__ cnt, int cap, unsigned* __restrict__ cmask,
                                                   int mw, int* __restrict__ ccnt, float wrap_margin, int wall_blocks,
                                                   int nwall, int nsys, const int* __restrict__ slot_of,
-                                                  PairRec* __restrict__ rec, const int* __restrict__ skip) {
+                                                  PairRec* __restrict__ rec, int* __restrict__ dense,
+                                                  const int* __restrict__ skip) {
     if (skip && *skip) return;
     if ((int)blockIdx.x < wall_blocks) {
         wall_velocity<ENS>(blockIdx.x * blockDim.x + threadIdx.x, nwall, n, p, s0, sys, nsys, slot_of, pos, vpred, vh,
@@ -692,6 +700,7 @@ __global__ void __launch_bounds__(kMaxBS, GC_DENS_MIN_BLOCKS) fk_density(int n, 
     const float4 vp = vpred[i];
     // 1/d - 1/d0 from the difference of the densities, which is exact where they are close
     const float z = p.rho0 > 0.f ? (p.rho0 - rho) * inv_d / p.rho0 : inv_d;
+    if (p.rho0 > 0.f && rho > kDense * p.rho0) *dense = 1;
     rec[i] = PairRec{xi4, make_float4(vp.x, vp.y, vp.z, z)};
 }
 
@@ -755,7 +764,8 @@ template <bool COMPACT, bool ENS, bool HALFV, bool NOISE, bool B1, int L, bool K
 __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
     fk_force(int n, GcParams p, SysInfo s0, const SysInfo* __restrict__ sys, const int* __restrict__ sysid,
              const unsigned* __restrict__ nkey, const PairRec* __restrict__ rec, const float4* __restrict__ pos,
-             const float4* __restrict__ vpred, const float2* __restrict__ dp, const float4* __restrict__ vh,
+             const float4* __restrict__ vpred, const float2* __restrict__ dp, const int* __restrict__ dense,
+             const float4* __restrict__ vh,
              float4* __restrict__ force, float4* __restrict__ vel, const int* __restrict__ nbr, const int* __restrict__ cnt, int cap,
              const unsigned* __restrict__ cmask, int mw, const float4* __restrict__ mforce, int drive,
              const uint2* __restrict__ vph, float wrap_margin, PhiloxKeys pk,
@@ -796,7 +806,7 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
         const float c2 = B1 ? (pid >= S.cs ? p.c2sq : p.c1sq) : p.c1sq;
         return (c2 * inv_d) * fmaf(-p.rho0, z, p.rest_m);
     };
-    constexpr bool apart = HALFV;   // gathers from the arrays instead of the records
+    const bool apart = HALFV || *dense;   // gathers from the arrays instead of the records
     const float idi = apart ? dp[i].x : p.rest_invd + vi.w;   // 1/d
     const float pti = apart ? dp[i].y : pterm(vi.w, idi, id);
     float2 fxy = make_float2(0.f, 0.f);
@@ -941,7 +951,12 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
             }
         }
     };
-    run_near<true>(axes, [&](auto w) { run(w, std::bool_constant<apart>{}); });
+    if constexpr (HALFV) {
+        run_near<true>(axes, [&](auto w) { run(w, std::true_type{}); });
+    } else {
+        if (apart) run(std::integral_constant<int, 7>{}, std::true_type{});
+        else run_near<true>(axes, [&](auto w) { run(w, std::false_type{}); });
+    }
     float3 f = f3(fxy.x, fxy.y, fz);
     if constexpr (L > 1) {
         const unsigned gm = group_mask<L>();
@@ -2110,7 +2125,7 @@ void density_launch(GcFused* f, cudaStream_t st, const GcParams& p, unsigned* cm
     auto go = [&](auto ens, auto b1) {
         fk_density<decltype(ens)::value, decltype(b1)::value, L><<<nb, bs, 0, st>>>(
             f->n, p, s0(f), f->dsys, f->a.sys, f->a.pos, f->a.vpred, f->a.vh, f->dp, f->nbr, f->cnt, f->cap, cm, f->mw,
-            cc, wrap_margin(f), wb, f->nwall, f->nsys, f->slot_of, f->rec, f->skip);
+            cc, wrap_margin(f), wb, f->nwall, f->nsys, f->slot_of, f->rec, f->rebuild + 1, f->skip);
     };
     if (f->ens) {
         if (f->has_b1) go(std::true_type{}, std::true_type{});
@@ -2169,7 +2184,7 @@ void force_launch_n(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
     for (int r = 0; r < 10; ++r) pk.k[r] = p.noise_key + 0x9E3779B9u * (unsigned)r;
     auto go = [&](auto ens, auto keys) {
         fk_force<COMPACT, decltype(ens)::value, HALFV, NOISE, B1, L, decltype(keys)::value><<<nb, f->block, 0, st>>>(
-            n, p, s0(f), f->dsys, f->a.sys, nk, f->rec, f->a.pos, f->a.vpred, f->dp, f->a.vh, f->a.force, f->a.vel, f->nbr, c, f->cap, cm,
+            n, p, s0(f), f->dsys, f->a.sys, nk, f->rec, f->a.pos, f->a.vpred, f->dp, f->rebuild + 1, f->a.vh, f->a.force, f->a.vel, f->nbr, c, f->cap, cm,
             f->mw, mf, drive, f->vph, wrap_margin(f), pk, f->skip);
     };
     if (f->ens) go(std::true_type{}, std::false_type{});
@@ -2303,7 +2318,7 @@ int one_step(GcFused* f, int drive) {
     GcParams p = f->p;
     p.noise_key = noise_key(p.seed, (uint64_t)f->step);
     if (f->ens) GC_TRY(launch_step_begin(f, st));
-    else GC_CUDA(cudaMemsetAsync(f->rebuild, 0, sizeof(int), st), "fused: flag");
+    else GC_CUDA(cudaMemsetAsync(f->rebuild, 0, 2 * sizeof(int), st), "fused: flag");
     GC_TRY(launch_integrate(f, st, p));
     const bool ahead = f->lists && !f->early && !f->profile && f->n < kAheadMost;
     cudaStream_t fs = ahead ? f->fst : st;
@@ -3174,7 +3189,7 @@ int gc_ensemble_create(int nsys, const GcSystemDesc* d, int noise_on, const GcFu
     if (ok == GC_OK) ok = falloc(f, &f->vals, n > f->ncp ? n : f->ncp);
     if (ok == GC_OK) ok = falloc(f, &f->cnt, n);
     if (ok == GC_OK) ok = falloc(f, &f->ccnt, n);
-    if (ok == GC_OK) ok = falloc(f, &f->rebuild, 1);
+    if (ok == GC_OK) ok = falloc(f, &f->rebuild, 2);
     if (ok == GC_OK) ok = falloc(f, &f->flags, 1);
     if (ok == GC_OK) ok = falloc(f, &f->oflag, 1);
     if (ok == GC_OK) ok = falloc(f, &f->need, 1);

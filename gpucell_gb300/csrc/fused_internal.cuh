@@ -235,7 +235,7 @@ struct GcFused {
     size_t cmask_elems = 0;
     int* ccnt = nullptr;         // number of acting entries
     int mw = 0;                  // mask words per slot
-    int* rebuild = nullptr;
+    int* rebuild = nullptr;      // the step's rebuild flag; and whether a particle is far above the rest density
     // pair tiles (GcFusedOptions.tiles): lists per pair of neighbouring
     // cubes built at each rebuild, partial sums per pair direction, finish
     // passes; otherwise per-particle Verlet lists for every slot

@@ -895,8 +895,8 @@ __global__ void __launch_bounds__(kMaxBS, L > 1 ? 4 : force_min_blocks(ENS))
         float cd = (pti + rj.pt) * F - (fdd * p.visB) * dv * ir2;
         add_f(-fdd * p.visA, vxy, vz);
         if constexpr (NOISE) {
-            // (a pair at the cut-off can give F a rounding-sized negative value: its noise is as small)
-            float q = sqrt_ftz(fabsf(p.noise_pref * fdd));
+            // (a pair at the cut-off can give F a rounding-sized negative value: no noise then)
+            float q = sqrt_ftz(fmaxf(p.noise_pref * fdd, 0.f));
             q = id < idj ? q : -q;   // the pair sign of xi_ij
             const unsigned ia = id - id0, ib = idj - id0;
             const Philox2 w = philox2x32_10_keys(min(ia, ib), max(ia, ib), [&](int r) {

@@ -405,8 +405,11 @@ __device__ __forceinline__ int scan_rows(int r0, int r1, int k, int i, float3 xi
 // even shares of the rows, count, and scan again to write each its part of
 // the list behind the parts before it (small systems, where a thread's serial
 // scan of 420 candidates sets the time: 102 us for 6 thousand particles, 56
-// with eight threads; from 80 thousand on two scans take longer than one).
+// with eight threads; a step with a build, with one and with eight: 16 thousand
+// particles 215 and 189 us, 32 thousand 253 and 256, 49 thousand 273 and 299).
 // The lists are the same entries in the same order either way.
+constexpr int kBuildLanesMost = 30000;
+
 template <int L>
 __global__ void __launch_bounds__(kMaxBS, kBuildMinBlocks) fk_build_list(int n, const SysInfo* __restrict__ sys,
                                                      const int* __restrict__ sysid, const float4* __restrict__ pos,
@@ -462,7 +465,7 @@ __global__ void __launch_bounds__(kMaxBS, kBuildMinBlocks) fk_build_list(int n, 
 // tiles.
 int launch_build(GcFused* f, cudaStream_t st, const float4* bpos, int walls_only) {
     const float cut = f->p.rc + f->skin;
-    const int L = f->lanes == 8 ? 8 : 1, nb = gc_blocks((long long)f->n * L, f->block);
+    const int L = f->n < kBuildLanesMost ? 8 : 1, nb = gc_blocks((long long)f->n * L, f->block);
     auto go = [&](auto kern) {
         kern<<<nb, f->block, 0, st>>>(f->n, f->dsys, f->a.sys, bpos, f->sb.cnt, f->nbr, f->cnt, f->cap, cut * cut,
                                       f->oflag, f->need, walls_only);
@@ -1432,22 +1435,6 @@ __device__ __forceinline__ void morse_pair(const GcParams& p, const GcGrid& g, f
     f += (fm * inv_r) * d;
 }
 
-// Candidates [a, b) of the cube-ordered arrays, four loads in flight.
-template <bool WRAP>
-__device__ __forceinline__ void morse_run(const GcParams& p, const GcGrid& g, float3 xi, float ai, unsigned a,
-                                          unsigned b, const float4* __restrict__ mspos,
-                                          const float* __restrict__ msarea, float3& f) {
-    unsigned s = a;
-    for (; s + 4 <= b; s += 4) {
-        float4 y0 = mspos[s], y1 = mspos[s + 1], y2 = mspos[s + 2], y3 = mspos[s + 3];
-        morse_pair<WRAP>(p, g, xi, ai, y0, msarea + s, f);
-        morse_pair<WRAP>(p, g, xi, ai, y1, msarea + s + 1, f);
-        morse_pair<WRAP>(p, g, xi, ai, y2, msarea + s + 2, f);
-        morse_pair<WRAP>(p, g, xi, ai, y3, msarea + s + 3, f);
-    }
-    for (; s < b; ++s) morse_pair<WRAP>(p, g, xi, ai, mspos[s], msarea + s, f);
-}
-
 // Morse aggregation by Verlet lists of its own.  When the neighbour lists
 // are rebuilt, each membrane vertex lists the vertices of other cells within
 // MaxCut + skin (no particle moves more than skin/2 before the next rebuild,
@@ -2306,11 +2293,12 @@ int passes(GcFused* f, const GcParams& p, int drive, bool hooks) {
 // step's passes again (the membrane passes run twice, with the same results).
 // The GPU then does not wait for the host in every step (15 us of a 90 us
 // step of a 6 thousand particle channel).  From kAheadMost particles on the
-// wait is below 3 % of a step and less than the passes queued twice cost (4.2 M
-// suspension: 4.17 ms a step waiting, 4.22 ahead; 524 k: 601 and 597 us; 350 k
-// sheared suspension: 549 and 532 us); steps with outputs written while they
-// run, with profiling marks and with the pair tiles wait too.
-constexpr int kAheadMost = 600000;
+// wait is less than the passes queued twice cost.  Red-cell suspensions, us a
+// step waiting / ahead: 524 k 587.7 / 586.8, 819 k 858.6 / 855.6, 1.18 M 1206 /
+// 1203, 1.6 M 1579 / 1579, 2.6 M 2556 / 2560, 4.2 M 4030 / 4047; a sheared
+// suspension of 350 k 549 / 532.  Steps with outputs written while they run,
+// with profiling marks and with the pair tiles wait too.
+constexpr int kAheadMost = 1500000;
 
 int one_step(GcFused* f, int drive) {
     cudaStream_t st = f->st;

@@ -65,7 +65,8 @@ __global__ void k_periodic(int n, GcParams p, const int* __restrict__ sortpart, 
         float v = *xs[a];
         if (v >= hi) { v -= L; *ts[a] += 1; }
         else if (v < lo) { v += L; *ts[a] -= 1; }
-        if (v >= hi || v < lo) raise_flag(flags, GC_FLAG_NONFINITE);
+        // less than half an ulp below lo, v + L rounds to hi itself: a position like any other
+        if (v > hi || v < lo) raise_flag(flags, GC_FLAG_NONFINITE);
         *xs[a] = v;
     }
     coor[i] = x;

@@ -284,12 +284,18 @@ def plain_bytes_per_step(cfg):
 # velocity, pressure and density read, force written) and the corrector of the
 # integration (28 B: VelHalf read, velocity written).
 FORCE_ALG_BYTES = 44 + 28
-# Bytes of the particle's own records fk_force moves: its position, predicted
-# velocity and VelHalf (16 B each) and (1/d, P/d^2) (8 B) read, force and
-# velocity (16 B each) written, the list length (4 B) read.  The neighbour
-# list entries it streams (4 B each) come on top: the Verlet lists are an
+# Bytes of the particle's own data fk_force moves: its pair record (32 B) and
+# VelHalf (16 B) read, force and velocity (16 B each) written, the number of
+# acting entries (4 B) read; and fk_density: position and predicted velocity
+# (16 B each) and the list length (4 B) read, (1/d, P/d^2) (8 B), the pair
+# record (32 B) and the number of acting entries (4 B) written.  The neighbour
+# list entries they stream (4 B each) come on top: the Verlet lists are an
 # implementation overhead of the fused step, not algorithmic bytes.
-FORCE_STATE_BYTES = 16 * 3 + 8 + 16 * 2 + 4
+FORCE_STATE_BYTES = 32 + 16 + 16 * 2 + 4
+DENSITY_STATE_BYTES = 16 * 2 + 4 + 8 + 32 + 4
+# The pair tiles' force passes read position, predicted velocity and (1/d, P/d^2)
+# instead of the record.
+TILE_STATE_BYTES = 16 * 3 + 8 + 16 * 2 + 4
 # Partial sums of the pair tiles per particle, written by the pair pass and
 # read back by its finish: 14 directions x 3 floats (force), x 1 (density).
 TILE_PARTIAL_BYTES = {"force": 2 * 14 * 12, "density": 2 * 14 * 4}
@@ -299,23 +305,24 @@ TILE_PARTIAL_BYTES = {"force": 2 * 14 * 12, "density": 2 * 14 * 4}
 # capture they come from):
 #   python bench.py --small --no-ensemble --cpu-steps 0 --no-plain --no-engine --no-output --no-parity
 #       --no-configs --no-variants --steps 3 --warmup 3 --profile-steps 1 --e2e-steps 1   (plain run, exit 0),
-#   then ncu --set full --clock-control none -k regex:"fk_(force|density)" -s 6 -c 2 <the same command>
+#   then ncu --set full --metrics sm__sass_thread_inst_executed_op_<op>_pred_on.sum (op: fadd, fmul, ffma, fadd2,
+#       fmul2, ffma2) --clock-control none -k regex:"fk_(force|density)" -s 6 -c 2 <the same command>
 # on the 524,288-particle suspension (warp instructions and FP32 operations
 # per particle; skin 0.125 rc, mean list 166.5), and
 #   ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum --clock-control none
 #       -k regex:"fk_(force|density|build_list|mgather|mgeo_edge|mtri|integrate)" -s 8 -c 8 python bench.py
 #       --no-ensemble --cpu-steps 0 --no-plain --no-engine --no-output --no-parity --no-configs --no-variants
 #       --steps 4 --warmup 3 --profile-steps 1 --e2e-steps 1
-# at full size (DRAM bytes of one launch, one pass).  The FP32 operations were
-# counted on the form without packed instructions, which do the same two at a
-# time.
+# at full size (DRAM bytes of one launch, one pass).  FP32 operations: 344.7 M
+# additions, 1109.6 M products, twice 1336.5 M multiply-adds and four times 56.7
+# M packed multiply-adds.
 FORCE_COUNTERS = {
     "kernel_version": "fk_force<1,0,0,1,0,1,1>: one thread per particle over its compact list of acting entries, "
-                      "32-byte neighbour records, packed FP32 pair terms, noise and wall-free forms as template "
-                      "switches",
-    "dram_bytes_per_launch_4M": 3.215104256e9 + 0.127953920e9,
-    "warp_inst_per_particle": 245566966 / 524288,
-    "fp32_flop_per_particle": 4.1227e9 / 524288,
+                      "32-byte neighbour records, packed velocity differences, noise and wall-free forms as "
+                      "template switches",
+    "dram_bytes_per_launch_4M": 3.215806720e9 + 0.128200192e9,
+    "warp_inst_per_particle": 245789225 / 524288,
+    "fp32_flop_per_particle": 4354121078 / 524288,
 }
 # SM schedulers of a GB300 (152 SMs x 4, one warp instruction per cycle
 # each) and its FP32 lanes (152 SMs x 128, an FMA counting 2).
@@ -361,17 +368,17 @@ def rooflines(cfg, ms_per_step, force_ms, dens_ms, mean_nb, hbm, peak_kind, cloc
     if tiles:
         # pair tiles: one 4-byte entry per candidate pair (mean_nb / 2 per
         # particle), 14 partial-sum planes written and read back by the finish
-        f_streamed = n * (FORCE_STATE_BYTES + TILE_PARTIAL_BYTES["force"] + 4 * mean_nb / 2)
+        f_streamed = n * (TILE_STATE_BYTES + TILE_PARTIAL_BYTES["force"] + 4 * mean_nb / 2)
         d_streamed = n * (24 + TILE_PARTIAL_BYTES["density"] + 4 * mean_nb / 2)
-        f_note = (f"streamed = {FORCE_STATE_BYTES} B of the particle's records + {TILE_PARTIAL_BYTES['force']} B of "
+        f_note = (f"streamed = {TILE_STATE_BYTES} B of the particle's records + {TILE_PARTIAL_BYTES['force']} B of "
                   f"partial sums per particle + 4 B per candidate pair ({mean_nb / 2:.1f} per particle)")
         d_note = (f"streamed = 24 + {TILE_PARTIAL_BYTES['density']} B of partial sums per particle + 4 B per "
                   "candidate pair")
     else:
         f_streamed = n * (FORCE_STATE_BYTES + 4 * mean_nb)
-        d_streamed = n * (24 + 4 * mean_nb)
+        d_streamed = n * (DENSITY_STATE_BYTES + 4 * mean_nb)
         f_note = f"streamed = {FORCE_STATE_BYTES} B per particle + 4 B per list entry (mean list {mean_nb:.1f})"
-        d_note = "streamed = 24 B per particle + 4 B per list entry"
+        d_note = f"streamed = {DENSITY_STATE_BYTES} B per particle + 4 B per list entry"
     kern = {
         "fk_force": {
             "launch_ms": force_ms, "bound": "hbm", "unit": "GB/s", "peak": hbm, "peak_source": peak_src,
@@ -406,7 +413,7 @@ def rooflines(cfg, ms_per_step, force_ms, dens_ms, mean_nb, hbm, peak_kind, cloc
         "kernel": "fk_force", "bound": "FP32 pipe", "unit": "TFLOP/s",
         "achieved": fpp * n / (force_ms / 1e3) / 1e12, "peak": GB300_FP32_FLOP_PER_CYCLE * mhz * 1e6 / 1e12,
         "frac": fpp * n / (force_ms / 1e3) / (GB300_FP32_FLOP_PER_CYCLE * mhz * 1e6),
-        "note": f"{fpp:.0f} FP32 operations per particle (FADD + FMUL + 2 FFMA, ncu); peak = 152 SMs x 128 lanes "
+        "note": f"{fpp:.0f} FP32 operations per particle (FADD + FMUL + 2 FFMA + 4 packed FMA, ncu); peak = 152 SMs x 128 lanes "
                 "x 2 x the sampled SM clock",
     }
     return roof, kern, issue, fp32

@@ -6,7 +6,10 @@ of independent systems shards with no data-path collective: the systems are
 assigned to ranks by longest-processing-time-first bin packing on their
 particle counts (the step cost is linear in particles), each rank steps its
 share as one ensemble, and only per-system results travel, gathered once at
-the end.
+the end.  A system draws the same noise on any rank, but its rounding depends
+on the systems it shares an ensemble with (list rebuilds, and the order of the
+sums, which follows from the ensemble's size): other distributions agree to
+rounding, not bit for bit.
 """
 from __future__ import annotations
 

@@ -295,7 +295,9 @@ int gc_fused_destroy(GcFused* f);
  * Many independent systems of uneven size stepped by the same launches: the
  * ids of system s follow those of systems 0..s-1, each system keeps its own
  * box, grid, body force (ConstExtForce) and noise seed (iSeed, keyed by the
- * system's own ids, so a system draws the same noise as when run alone);
+ * system's own ids, so a system draws the same noise as when run alone; its
+ * rounding depends on the others, which share its list rebuilds and whose
+ * number of particles decides the order of the sums);
  * every other Structconst field must be the same for all systems.  A handle
  * from gc_ensemble_create takes the gc_fused_* calls too: gc_fused_load,
  * _store, _store_cells and _cell_sums then cover all systems, concatenated in

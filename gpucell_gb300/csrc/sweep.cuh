@@ -155,10 +155,24 @@ __device__ __forceinline__ int form_of(float3 x, const Limits& l, float3 lim) {
     return d.x < kFar && d.y < kFar && d.z < kFar ? 7 : kAny;
 }
 
+// Difference along an axis; with IMAGE the minimum image, the same as
+// min_image_1's (half: half the box, infinite along wall axes).  One comparison
+// instead of two per axis: the cubes at the faces are the last blocks to end in a
+// small box (density of 13.8 thousand particles 66 -> 52 us, 614 thousand 471 -> 456).
 template <bool IMAGE>
-__device__ __forceinline__ float3 diff(float3 a, float4 b, const GcGrid& g) {
-    if constexpr (IMAGE) return min_image(a, f3(b.x, b.y, b.z), g);
-    else return f3(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y), __fsub_rn(a.z, b.z));
+__device__ __forceinline__ float diff_1(float a, float b, float half, float L) {
+    const float d = __fsub_rn(a, b);
+    return IMAGE && fabsf(d) > half ? __fsub_rn(d, copysignf(L, d)) : d;
+}
+
+template <bool IMAGE>
+__device__ __forceinline__ float3 diff(float3 a, float4 b, float3 half, const GcGrid& g) {
+    return f3(diff_1<IMAGE>(a.x, b.x, half.x, g.L[0]), diff_1<IMAGE>(a.y, b.y, half.y, g.L[1]),
+              diff_1<IMAGE>(a.z, b.z, half.z, g.L[2]));
+}
+
+__device__ __forceinline__ float3 half_box(const GcGrid& g) {
+    return f3(g.pmask & 1 ? g.halfL[0] : INFINITY, g.pmask & 2 ? g.halfL[1] : INFINITY, g.pmask & 4 ? g.halfL[2] : INFINITY);
 }
 
 // Marks the staged candidates [0, m) (m a multiple of 4 kGroup, padded with
@@ -175,6 +189,7 @@ template <int FORM>
 __device__ __forceinline__ int mark(Shared& sh, float3 xa, float3 xb, int s, int m, float cutm, const GcGrid& g) {
     const float3 L = f3(g.pmask & 1 ? g.L[0] : INFINITY, g.pmask & 2 ? g.L[1] : INFINITY,
                         g.pmask & 4 ? g.L[2] : INFINITY);
+    const float3 half = half_box(g);
     auto beyond = [&](float3 x, float4 y) {
         float dx = __fsub_rn(x.x, y.x), dy = __fsub_rn(x.y, y.y), dz = __fsub_rn(x.z, y.z);
         if constexpr (FORM & 1) dx = fminf(fabsf(dx), L.x - fabsf(dx));
@@ -193,8 +208,8 @@ __device__ __forceinline__ int mark(Shared& sh, float3 xa, float3 xb, int s, int
                 const float4 xj = x[(u0 + u) * kGroup];
                 if constexpr (FORM == kAny) {
                     const bool none = xj.x == kFar;
-                    a = (a << 1) | (none || norm2_rn(diff<true>(xa, xj, g)) >= cutm ? 0u : 1u);
-                    b = (b << 1) | (none || norm2_rn(diff<true>(xb, xj, g)) >= cutm ? 0u : 1u);
+                    a = (a << 1) | (none || norm2_rn(diff<true>(xa, xj, half, g)) >= cutm ? 0u : 1u);
+                    b = (b << 1) | (none || norm2_rn(diff<true>(xb, xj, half, g)) >= cutm ? 0u : 1u);
                 } else {
                     a = __funnelshift_l(__float_as_uint(beyond(xa, xj)), a, 1);
                     b = __funnelshift_l(__float_as_uint(beyond(xb, xj)), b, 1);
@@ -251,6 +266,7 @@ __device__ __forceinline__ void evaluate(const Op& op, const typename Op::Extra&
     }
     for (; r > 0; --r) bits &= ~(0x80000000u >> __clz(bits));   // the bit
     const int words = (m + kWord - 1) / kWord;
+    const float3 half = half_box(p.g);
     for (; n > 0; --n) {
         while (!bits) {   // ends: n marks are left
             if (++w == words) {
@@ -263,7 +279,7 @@ __device__ __forceinline__ void evaluate(const Op& op, const typename Op::Extra&
         bits &= ~(0x80000000u >> u);
         const int q = w * kWord + u * kGroup + lane;
         const float4 xj = sh.x[q];
-        const float3 d = diff<IMAGE>(xi, xj, p.g);
+        const float3 d = diff<IMAGE>(xi, xj, half, p.g);
         const float r2 = norm2_rn(d);
         if (!(r2 >= cut2)) op.pair(acc, self, ex, q, __float_as_uint(xj.w), d, r2, p);
     }

@@ -177,8 +177,8 @@ __global__ void k_eos(int n, GcParams p, const int* __restrict__ sortpart, const
 // and the e e^T parts of the viscous and random forces, e = d/r), one along
 // v_ij and one along xi_ij, as in the fused step.  Roots and divisions are the
 // correctly rounded ones, here and in the other sweeps: with rsqrt.approx and
-// a product of two reciprocals a million-particle step took 3.06 instead of
-// 3.24 ms, but a pair near the cut-off, where F goes as (1 - r/rc)^3, was off
+// a product of two reciprocals a million-particle step took 0.18 ms less (3.06
+// of 3.24), but a pair near the cut-off, where F goes as (1 - r/rc)^3, was off
 // by twice as much.
 template <bool NOISE>
 struct SdpdOp {

@@ -14,11 +14,11 @@
 // thousand particle channel is 650 blocks of one thread per particle, each a
 // serial chain of 750 candidates.
 //
-// Bound by instruction issue (79 % of the slots in the density sweep, 71 % in
+// Bound by instruction issue (81 % of the slots in the density sweep, 72 % in
 // the SDPD sweep, where shared memory holds six blocks a SM).  Measured on
-// one GB300: a million-particle suspension's step 6.73 -> 3.25 ms, an 83
-// thousand particle channel with walls of both kinds 1.55 -> 0.44 ms; at 524
-// thousand particles the density sweep takes 0.41 ms and the SDPD sweep 0.80
+// one GB300: a million-particle suspension's step 6.73 -> 3.16 ms, an 83
+// thousand particle channel with walls of both kinds 1.55 -> 0.42 ms; at 524
+// thousand particles the density sweep takes 0.39 ms and the SDPD sweep 0.75
 // (2.50 before).  On an earlier form of it, 0.66 and 1.32 ms for a million
 // particles, one particle per four lanes testing for itself took 0.86 and 1.51
 // ms (a shared-memory load per test), without even shares 0.99 and 2.26 ms.

@@ -1460,7 +1460,8 @@ __device__ __forceinline__ void morse_pair(const GcParams& p, const GcGrid& g, f
 // only the listed pairs.
 //
 // The list build (fk_mlist) runs a warp per vertex over the (2R+1)^3
-// aggregation cubes around it (agg_grid: the stencil reaches MaxCut + skin).  The lanes test 32 cubes at a time (cubes
+// aggregation cubes around it (agg_grid: the stencil reaches MaxCut + skin).
+// The lanes test 32 cubes at a time (cubes
 // farther than the cut-off are not read) and then go through each cube that
 // is left together, lane k taking the candidates k, k + 32, ...: consecutive
 // loads and no lane waiting for another.  A first pass counts, a scan places
@@ -1938,9 +1939,11 @@ int agg_grid(const float* bbox, float maxcut, float cutl, int mask, GcGrid* g, i
                (!(mask & 2) || g->n[1] >= 5) && (!(mask & 4) || g->n[2] >= 5);
     };
     if (!half_width(maxcut)) GC_TRY(gc_build_grid(bbox, maxcut, mask, g));
+    const GcGrid box = *g;
     *R = 2;
     if (half_width(cutl)) return GC_OK;
     *R = 1;
+    *g = box;   // an attempt that fails leaves it half filled
     g->ncells = 1;
     for (int a = 0; a < 3; ++a) {
         const bool per = (mask >> a) & 1;
@@ -2189,8 +2192,8 @@ void force_launch_n(GcFused* f, cudaStream_t st, const GcParams& p, int drive) {
     for (int r = 0; r < 10; ++r) pk.k[r] = p.noise_key + 0x9E3779B9u * (unsigned)r;
     auto go = [&](auto ens, auto keys) {
         fk_force<COMPACT, decltype(ens)::value, HALFV, NOISE, B1, L, decltype(keys)::value><<<nb, f->block, 0, st>>>(
-            n, p, s0(f), f->dsys, f->a.sys, nk, f->rec, f->a.pos, f->a.vpred, f->dp, f->rebuild + 1, f->a.vh, f->a.force, f->a.vel, f->nbr, c, f->cap, cm,
-            f->mw, mf, drive, f->vph, wrap_margin(f), pk, f->skip);
+            n, p, s0(f), f->dsys, f->a.sys, nk, f->rec, f->a.pos, f->a.vpred, f->dp, f->rebuild + 1, f->a.vh,
+            f->a.force, f->a.vel, f->nbr, c, f->cap, cm, f->mw, mf, drive, f->vph, wrap_margin(f), pk, f->skip);
     };
     if (f->ens) go(std::true_type{}, std::false_type{});
     else if (NOISE && !nk) go(std::false_type{}, std::bool_constant<NOISE>{});

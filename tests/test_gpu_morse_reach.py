@@ -56,3 +56,32 @@ def test_pairs_that_approach_are_listed(cuda_device, axis, cubes):
     np.testing.assert_allclose(g["AggForce"], o.aggforce, rtol=0, atol=1e-3 * scale)
     assert fs.flags() == 0
     fs.close()
+
+
+@pytest.mark.parametrize("box, skin", [((10.01, 12.0, 11.0), 1.0), ((7.6, 9.0, 7.7), 0.3)])
+def test_boxes_of_few_cubes(cuda_device, box, skin):
+    """Boxes that take MaxCut, or five times half of it, along every axis but not
+    MaxCut + skin."""
+    from gpucell_gb300.fused import FusedSystem
+    from oracle.binding import Oracle
+    max_cut = 4.0 if box[0] > 10 else 2.5
+    rng = np.random.default_rng(2)
+    verts, faces = gen.icosphere(1)
+    cells = [(1.2 * verts + rng.uniform(0, 1, 3) * box, faces) for _ in range(6)]
+    none = np.zeros((0, 3))
+    phys = gen.Physics(ext_force=0.0, dt=1e-6, sur_energy=5.0, max_cut=max_cut, zero_len=0.3, sca_fac=1.5)
+    cfg = gen._assemble("few", np.stack([np.zeros(3), box], 1).ravel(), 7, none, none, rng.uniform(0, 1, (500, 3)) * box,
+                        cells, phys, 1.0 / 3.0)
+    o = Oracle(cfg, noise=False)
+    o.setup()
+    fs = FusedSystem(cfg, noise=False, skin=skin)
+    for _ in range(2):
+        o.step()
+    fs.step(2, 1)
+    g = fs.fetch()
+    scale = np.abs(o.aggforce).max()
+    assert scale > 0
+    # sums of up to 200 FP32 terms of a few roundings each, as for the cells of the other tests
+    np.testing.assert_allclose(g["AggForce"], o.aggforce, rtol=0, atol=2e-5 * scale)
+    assert fs.flags() == 0
+    fs.close()
